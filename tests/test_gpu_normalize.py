@@ -68,3 +68,33 @@ def test_normalize_without_gate_and_refused_branches():
         normalize_gate_fn(xc, residual=xc)
     with pytest.raises(AssertionError):
         normalize_gate_fn(xc, gate=xc, gate_act="softmax")
+
+
+@pytest.mark.parametrize("use_mean,pos", [(False, "pre"), (True, "post"), (True, "pre")])
+@pytest.mark.parametrize("offset", [0, 4])
+@pytest.mark.parametrize("e", [4, 36, 64, 72, 136, 256, 264, 512])
+def test_normalize_gate_lane_splits(e, offset, use_mean, pos):
+    """Every split of a group over lanes (8, 16, 32 lanes, one or more packs of 8 or 4 features), a row
+    count that is no multiple of a warp's rows, and tensors that start 8 bytes off a 16-byte boundary."""
+    from xopes_b200.normalize import normalize_gate_fn
+    gen = torch.Generator().manual_seed(e)
+    groups, rows = 3, 77
+    n = rows * groups * e
+
+    def make(t):  # the same values, `offset` elements into a larger buffer
+        buf = torch.zeros(n + offset, dtype=torch.bfloat16, device="cuda")
+        buf[offset:] = t.reshape(-1).to(torch.bfloat16).cuda()
+        return buf[offset:].view(rows, groups * e)
+
+    x, gate, do = (torch.randn(rows, groups * e, generator=gen).bfloat16().float() for _ in range(3))
+    w, b = 1 + 0.1 * torch.randn(groups * e, generator=gen), 0.1 * torch.randn(groups * e, generator=gen)
+    xc, gc = make(x).requires_grad_(), make(gate).requires_grad_()
+    wc, bc = w.cuda().requires_grad_(), b.cuda().requires_grad_()
+    o = normalize_gate_fn(xc, wc, bc, gate=gc, gate_act="silu", gate_pos=pos, c=e ** 0.5, use_mean=use_mean,
+                          num_groups=groups)
+    g = torch.autograd.grad(o, [xc, gc, wc, bc], make(do))
+    xr, gr, wr, br = (t.clone().requires_grad_() for t in (x, gate, w, b))
+    ro = norc.normalize_gate(xr, wr, br, gr, "silu", pos, e ** 0.5, 1e-6, use_mean, groups)
+    rg = torch.autograd.grad((ro * do.double()).sum(), [xr, gr, wr, br])
+    for name, ref, got in zip(("o", "dx", "dgate", "dweight", "dbias"), (ro,) + rg, (o,) + g):
+        assert_close(name, ref.float(), got.float(), TOL_BF16)

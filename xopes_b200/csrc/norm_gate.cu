@@ -8,46 +8,50 @@
 //   o  = y            (gate_pos = pre, or no gate)   or   y (.) a   (gate_pos = post)
 //
 // One pass over x and gate in, o out (forward), and one pass over x, gate, do in, dx, dgate out
-// (backward), all arithmetic in fp32: pure HBM streaming, 3 x 2e bytes per group forward.  One warp
-// owns one (row, group) at a time, a lane owns e / 32 elements as packs of 4; a warp walks rows of
-// ONE group, so the weight / bias gradients accumulate in registers and leave with one atomicAdd
-// per lane and element at the end.
+// (backward), all arithmetic in fp32: pure HBM streaming, 3 x 2e bytes per group forward and
+// 5 x 2e backward.  LPG lanes own one (row, group) at a time, so a warp works on 32 / LPG rows of ONE
+// group; the weight / bias gradients accumulate in registers, meet in shared memory once at the
+// end and leave with one atomicAdd per feature and CTA.
 #include "common.cuh"
 
 namespace la {
 namespace {
 
-constexpr int kMaxPerLane = 16;  // e <= 512
+constexpr int kMaxFeatures = 512;
+constexpr int kThreads = 256, kWarps = kThreads / 32;
 
 enum { kActNone = 0, kActRelu = 1, kActSigmoid = 2, kActSilu = 3 };
 
-__device__ __forceinline__ float act_f(float g, int act) {
-  switch (act) {
-    case kActRelu: return fmaxf(g, 0.f);
-    case kActSigmoid: return 1.f / (1.f + __expf(-g));
-    case kActSilu: return g / (1.f + __expf(-g));
-  }
-  return g;
-}
-// derivative of the activation at g
-__device__ __forceinline__ float act_grad(float g, int act) {
-  switch (act) {
-    case kActRelu: return g >= 0.f ? 1.f : 0.f;
-    case kActSigmoid: {
-      const float s = 1.f / (1.f + __expf(-g));
-      return s * (1.f - s);
+// act[j] = activation of g[j]; dact[j] = its derivative (only when asked for).  The activation is
+// the same for the whole launch, so the choice is a branch around the loops.
+template <bool GRAD, int N>
+__device__ __forceinline__ void activate(const float (&g)[N], int kind, float (&act)[N], float (&dact)[N]) {
+  if (kind == kActSigmoid || kind == kActSilu) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const float s = 1.f / (1.f + __expf(-g[j]));
+      if (kind == kActSigmoid) {
+        act[j] = s;
+        if (GRAD) dact[j] = s * (1.f - s);
+      } else {
+        act[j] = g[j] * s;
+        if (GRAD) dact[j] = s * (1.f + g[j] * (1.f - s));
+      }
     }
-    case kActSilu: {
-      const float s = 1.f / (1.f + __expf(-g));
-      return s * (1.f + g * (1.f - s));
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      act[j] = kind == kActRelu ? fmaxf(g[j], 0.f) : g[j];
+      if (GRAD) dact[j] = (kind == kActRelu && !(g[j] >= 0.f)) ? 0.f : 1.f;
     }
   }
-  return 1.f;
 }
 
-__device__ __forceinline__ float warp_sum(float v) {
+// sum over the LPG consecutive lanes that share a (row, group)
+template <int LPG>
+__device__ __forceinline__ float lane_sum(float v) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  for (int off = LPG / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
 }
 
@@ -63,183 +67,242 @@ struct NormArgs {
   float c, eps;
 };
 
-// Loads this lane's elements of one group: element j of the lane is feature lane * 4 + (j / 4) * 128 + j % 4.
-template <typename T, int N>
-__device__ __forceinline__ void load_lane(const T *p, int e, int lane, float (&v)[N]) {
+// VEC consecutive elements of type T as one aligned access.
+template <int BYTES> struct Raw;
+template <> struct Raw<16> { typedef uint4 type; };
+template <> struct Raw<8> { typedef uint2 type; };
+template <typename T, int VEC> struct Pack {
+  typedef typename Raw<VEC * (int)sizeof(T)>::type R;
+  static __device__ __forceinline__ void unpack(const R &raw, float *v) {
+    const T *h = reinterpret_cast<const T *>(&raw);
 #pragma unroll
-  for (int j = 0; j < N; j += 4) {
-    {
-      const int f = lane * 4 + (j >> 2) * 128;
-      if (f < e) {
-        if (sizeof(T) == 2) {
-          const uint2 u = *reinterpret_cast<const uint2 *>(p + f);
-          const T *h = reinterpret_cast<const T *>(&u);
-          v[j] = Cvt<T>::to_f(h[0]); v[j + 1] = Cvt<T>::to_f(h[1]); v[j + 2] = Cvt<T>::to_f(h[2]); v[j + 3] = Cvt<T>::to_f(h[3]);
-        } else {
-          const float4 u = *reinterpret_cast<const float4 *>(p + f);
-          v[j] = u.x; v[j + 1] = u.y; v[j + 2] = u.z; v[j + 3] = u.w;
-        }
-      } else {
-        v[j] = v[j + 1] = v[j + 2] = v[j + 3] = 0.f;
-      }
-    }
+    for (int j = 0; j < VEC; ++j) v[j] = Cvt<T>::to_f(h[j]);
   }
-}
-template <typename T, int N>
-__device__ __forceinline__ void store_lane(T *p, int e, int lane, const float (&v)[N]) {
+  static __device__ __forceinline__ R pack(const float *v) {
+    R raw;
+    T *h = reinterpret_cast<T *>(&raw);
 #pragma unroll
-  for (int j = 0; j < N; j += 4) {
-    {
-      const int f = lane * 4 + (j >> 2) * 128;
-      if (f < e) {
-        if (sizeof(T) == 2) {
-          T h[4] = {Cvt<T>::from_f(v[j]), Cvt<T>::from_f(v[j + 1]), Cvt<T>::from_f(v[j + 2]), Cvt<T>::from_f(v[j + 3])};
-          *reinterpret_cast<uint2 *>(p + f) = *reinterpret_cast<const uint2 *>(h);
-        } else {
-          *reinterpret_cast<float4 *>(p + f) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        }
-      }
-    }
+    for (int j = 0; j < VEC; ++j) h[j] = Cvt<T>::from_f(v[j]);
+    return raw;
   }
+};
+
+// resident CTAs per SM without spills (N = features per lane)
+template <bool BWD, bool POST, int N> constexpr int ctas_per_sm() {
+  return N <= (BWD && POST ? 4 : 8) ? 3 : (N <= 8 ? 2 : 1);
 }
 
-// grid (blocks over rows, G); a warp takes rows blockIdx.x * warps + warp, then strides.
-// N = elements per lane = 4 * ceil(e / 128).
-template <typename T, bool BWD, int N>
-__global__ void __launch_bounds__(256) norm_gate_kernel(const NormArgs a) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+// Grid (CTAs over rows, G).  Lane l of the LPG lanes of a (row, group) owns NP packs of VEC features,
+// pack p being features [(p LPG + l) VEC, +VEC); packs past e are zero.  The rows of a warp's next
+// step are loaded before the current step is worked on.
+//
+// Bound by HBM: 75 MB forward / 126 MB backward at 16384 rows of 12 groups of 64 (bf16) are 11.5 / 19 us
+// at the measured copy bandwidth.  A whole warp per group left half its lanes idle at 64 features,
+// had one 8-byte load per operand in flight and sent one atomic per warp and feature.
+//
+// POST = false: no gate behind the norm (the backward then needs neither y nor the bias, which is
+// what lets a third CTA onto the SM).
+template <typename T, bool BWD, bool POST, int VEC, int LPG, int NP>
+__global__ void __launch_bounds__(kThreads, (ctas_per_sm<BWD, POST, VEC * NP>())) norm_gate_kernel(const NormArgs a) {
+  typedef Pack<T, VEC> P;
+  typedef typename P::R R;
+  constexpr int N = VEC * NP, RPW = 32 / LPG;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gl = lane % LPG, sub = lane / LPG;
   const int g = blockIdx.y, e = a.e;
   const long long stride = (long long)a.G * e;
   const bool has_gate = a.gate != nullptr;
   float w[N], b[N], dw[N], db[N];
 #pragma unroll
-  for (int j = 0; j < N; ++j) { w[j] = 1.f; b[j] = 0.f; dw[j] = 0.f; db[j] = 0.f; }
-  if (a.weight != nullptr) load_lane<float, N>(a.weight + (long long)g * e, e, lane, w);
-  if (a.bias != nullptr) load_lane<float, N>(a.bias + (long long)g * e, e, lane, b);
-  const float inv_e = 1.f / (float)e;
-
-  for (long long r = (long long)blockIdx.x * warps + warp; r < a.rows; r += (long long)gridDim.x * warps) {
-    const long long off = r * stride + (long long)g * e;
-    float x[N], gt[N], act[N], z[N];
-    load_lane<T, N>(static_cast<const T *>(a.x) + off, e, lane, x);
-    if (has_gate) load_lane<T, N>(static_cast<const T *>(a.gate) + off, e, lane, gt);
-    float s1 = 0.f;
+  for (int p = 0; p < NP; ++p)
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      {
-        act[j] = has_gate ? act_f(gt[j], a.act) : 1.f;
-        z[j] = (has_gate && !a.post) ? x[j] * act[j] : x[j];
-        s1 += z[j];
-      }
+    for (int j = 0; j < VEC; ++j) {
+      const int f = (p * LPG + gl) * VEC + j, i = p * VEC + j;
+      w[i] = (a.weight != nullptr && f < e) ? a.weight[(long long)g * e + f] : 1.f;
+      b[i] = ((POST || !BWD) && a.bias != nullptr && f < e) ? a.bias[(long long)g * e + f] : 0.f;
+      dw[i] = db[i] = 0.f;
     }
-    float mean = 0.f;
-    if (a.use_mean) mean = warp_sum(s1) * inv_e;
-    float s2 = 0.f;
+  const float inv_e = 1.f / (float)e;
+  const T *xp = static_cast<const T *>(a.x), *gp = static_cast<const T *>(a.gate), *dp = static_cast<const T *>(a.d_out);
+  const long long step = (long long)gridDim.x * kWarps * RPW;
+  R rx[NP], rg[NP], rd[NP];
+  const R zero = {};
+  auto fetch = [&](long long r) {
+    const long long off = r * stride + (long long)g * e;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int f = (p * LPG + gl) * VEC;
+      const bool on = r < a.rows && f < e;
+      rx[p] = on ? *reinterpret_cast<const R *>(xp + off + f) : zero;
+      rg[p] = (on && has_gate) ? *reinterpret_cast<const R *>(gp + off + f) : zero;
+      if (BWD) rd[p] = on ? *reinterpret_cast<const R *>(dp + off + f) : zero;
+    }
+  };
+  const long long first = ((long long)blockIdx.x * kWarps + warp) * RPW;  // uniform over the warp
+  fetch(first + sub);
+  for (long long r0 = first; r0 < a.rows; r0 += step) {
+    const long long r = r0 + sub;
+    const bool live = r < a.rows;
+    const long long off = r * stride + (long long)g * e;
+    float x[N], gt[N], d_o[N], act[N], dact[N], z[N];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      P::unpack(rx[p], x + p * VEC);
+      P::unpack(rg[p], gt + p * VEC);
+      if (BWD) P::unpack(rd[p], d_o + p * VEC);
+    }
+    fetch(r + step);
+    if (has_gate) {
+      activate<BWD, N>(gt, a.act, act, dact);
+    } else {
+#pragma unroll
+      for (int j = 0; j < N; ++j) { act[j] = 1.f; dact[j] = 0.f; }
+    }
+    const bool pre = has_gate && !a.post, post = POST && has_gate && a.post;
+    float s1 = 0.f, s2 = 0.f, mean = 0.f;
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      {
-        const int f = lane * 4 + (j >> 2) * 128 + (j & 3);
-        z[j] = f < e ? z[j] - mean : 0.f;  // zc
+      z[j] = pre ? x[j] * act[j] : x[j];
+      s1 += z[j];
+    }
+    if (a.use_mean) mean = lane_sum<LPG>(s1) * inv_e;
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int j = p * VEC; j < (p + 1) * VEC; ++j) {
+        z[j] = (p * LPG + gl) * VEC < e ? z[j] - mean : 0.f;  // zc (e is a multiple of VEC)
         s2 += z[j] * z[j];
       }
-    }
-    const float rsig = rsqrtf(warp_sum(s2) + a.eps);
+    const float rsig = rsqrtf(lane_sum<LPG>(s2) + a.eps);
     if (!BWD) {
       float o[N];
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        {
-          const float y = a.c * z[j] * rsig * w[j] + b[j];
-          o[j] = (has_gate && a.post) ? y * act[j] : y;
-        }
+        const float y = a.c * z[j] * rsig * w[j] + b[j];
+        o[j] = post ? y * act[j] : y;
       }
-      store_lane<T, N>(static_cast<T *>(a.out) + off, e, lane, o);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const int f = (p * LPG + gl) * VEC;
+        if (live && f < e) *reinterpret_cast<R *>(static_cast<T *>(a.out) + off + f) = P::pack(o + p * VEC);
+      }
     } else {
-      float d_o[N], dxh[N], dga[N];
-      load_lane<T, N>(static_cast<const T *>(a.d_out) + off, e, lane, d_o);
+      float dxh[N], dga[N];
       float dot = 0.f;
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        {
-          const float xh = z[j] * rsig;                    // normalised value
-          const float y = a.c * xh * w[j] + b[j];
-          const float dy = (has_gate && a.post) ? d_o[j] * act[j] : d_o[j];
-          dga[j] = (has_gate && a.post) ? d_o[j] * y : 0.f;  // d loss / d act(gate), post-gate part
-          dw[j] += dy * a.c * xh;
-          db[j] += dy;
-          dxh[j] = dy * w[j] * a.c;
-          dot += dxh[j] * xh;
-        }
+        const float xh = z[j] * rsig;                    // normalised value
+        const float y = a.c * xh * w[j] + b[j];
+        const float dy = post ? d_o[j] * act[j] : d_o[j];
+        dga[j] = post ? d_o[j] * y : 0.f;                // d loss / d act(gate), post-gate part
+        dw[j] += dy * a.c * xh;                          // rows past the end add zero: do reads as zero there
+        db[j] += dy;
+        dxh[j] = dy * w[j] * a.c;
+        dot += dxh[j] * xh;
       }
-      dot = warp_sum(dot);
+      dot = lane_sum<LPG>(dot);
       float s3 = 0.f;
 #pragma unroll
-      for (int j = 0; j < N; ++j) {
-        {
-          const int f = lane * 4 + (j >> 2) * 128 + (j & 3);
+      for (int p = 0; p < NP; ++p)
+#pragma unroll
+        for (int j = p * VEC; j < (p + 1) * VEC; ++j) {
           const float xh = z[j] * rsig;
-          dxh[j] = f < e ? (dxh[j] - xh * dot) * rsig : 0.f;  // d loss / d zc
+          dxh[j] = (p * LPG + gl) * VEC < e ? (dxh[j] - xh * dot) * rsig : 0.f;  // d loss / d zc
           s3 += dxh[j];
         }
-      }
       float dmean = 0.f;
-      if (a.use_mean) dmean = warp_sum(s3) * inv_e;
+      if (a.use_mean) dmean = lane_sum<LPG>(s3) * inv_e;
       float gx[N], gg[N];
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        {
-          const float dz = dxh[j] - dmean;                 // d loss / d z
-          if (has_gate && !a.post) {
-            gx[j] = dz * act[j];
-            dga[j] = dz * x[j];
-          } else {
-            gx[j] = dz;
-          }
-          gg[j] = has_gate ? dga[j] * act_grad(gt[j], a.act) : 0.f;
+        const float dz = dxh[j] - dmean;                 // d loss / d z
+        gx[j] = pre ? dz * act[j] : dz;
+        if (pre) dga[j] = dz * x[j];
+        gg[j] = dga[j] * dact[j];
+      }
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const int f = (p * LPG + gl) * VEC;
+        if (live && f < e) {
+          *reinterpret_cast<R *>(static_cast<T *>(a.dx) + off + f) = P::pack(gx + p * VEC);
+          if (has_gate) *reinterpret_cast<R *>(static_cast<T *>(a.dgate) + off + f) = P::pack(gg + p * VEC);
         }
       }
-      store_lane<T, N>(static_cast<T *>(a.dx) + off, e, lane, gx);
-      if (has_gate) store_lane<T, N>(static_cast<T *>(a.dgate) + off, e, lane, gg);
     }
   }
-  if (BWD) {
+  if (BWD && (a.dweight != nullptr || a.dbias != nullptr)) {  // uniform over the grid
+    __shared__ float part[2][kWarps][LPG * N];
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      {
-        const int f = lane * 4 + (j >> 2) * 128 + (j & 3);
-        if (f < e) {
-          if (a.dweight != nullptr) atomicAdd(a.dweight + (long long)g * e + f, dw[j]);
-          if (a.dbias != nullptr) atomicAdd(a.dbias + (long long)g * e + f, db[j]);
-        }
+#pragma unroll
+      for (int o = LPG; o < 32; o <<= 1) {
+        dw[j] += __shfl_xor_sync(0xffffffffu, dw[j], o);
+        db[j] += __shfl_xor_sync(0xffffffffu, db[j], o);
       }
+      const int f = ((j / VEC) * LPG + gl) * VEC + j % VEC;
+      if (sub == 0) {
+        part[0][warp][f] = dw[j];
+        part[1][warp][f] = db[j];
+      }
+    }
+    __syncthreads();
+    for (int f = threadIdx.x; f < e; f += kThreads) {
+      float sw = 0.f, sb = 0.f;
+#pragma unroll
+      for (int k = 0; k < kWarps; ++k) {
+        sw += part[0][k][f];
+        sb += part[1][k][f];
+      }
+      if (a.dweight != nullptr) atomicAdd(a.dweight + (long long)g * e + f, sw);
+      if (a.dbias != nullptr) atomicAdd(a.dbias + (long long)g * e + f, sb);
     }
   }
 }
 
-template <typename T>
-int launch_t(const NormArgs &a, bool bwd, cudaStream_t st) {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+template <typename T, int VEC, int LPG, int NP>
+int launch_cfg(const NormArgs &a, bool bwd, cudaStream_t st) {
+  static int sms[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LA_ERR_CUDA;
+  if (sms[dev] == 0 && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return LA_ERR_CUDA;
-  const int warps = 8;
-  long long blocks = (a.rows + warps - 1) / warps;
-  // enough CTAs to fill the GPU several times over, few enough that the per-warp gradient
-  // accumulators are flushed rarely
-  const long long cap = (long long)sms * 8 / (a.G > 0 ? (a.G < 8 ? a.G : 8) : 1) + 1;
+  const long long rows_per_cta = (long long)kWarps * (32 / LPG);
+  long long blocks = (a.rows + rows_per_cta - 1) / rows_per_cta;
+  // one wave over all groups: each CTA ends with its gradient sums, so few CTAs that walk many rows
+  const bool post = a.gate != nullptr && a.post;
+  const int resident = !bwd ? ctas_per_sm<false, true, VEC * NP>()
+                            : (post ? ctas_per_sm<true, true, VEC * NP>() : ctas_per_sm<true, false, VEC * NP>());
+  const long long cap = ((long long)sms[dev] * resident + a.G - 1) / a.G;
   if (blocks > cap) blocks = cap;
   dim3 grid((unsigned)blocks, (unsigned)a.G);
-  const int n = ((a.e + 127) / 128) * 4;
-#define LA_NORM_LAUNCH(NN)                                                            \
-  do {                                                                                \
-    if (bwd) norm_gate_kernel<T, true, NN><<<grid, warps * 32, 0, st>>>(a);           \
-    else norm_gate_kernel<T, false, NN><<<grid, warps * 32, 0, st>>>(a);              \
-  } while (0)
-  if (n <= 4) LA_NORM_LAUNCH(4);
-  else if (n <= 8) LA_NORM_LAUNCH(8);
-  else LA_NORM_LAUNCH(16);
-#undef LA_NORM_LAUNCH
+  if (!bwd) norm_gate_kernel<T, false, true, VEC, LPG, NP><<<grid, kThreads, 0, st>>>(a);
+  else if (post) norm_gate_kernel<T, true, true, VEC, LPG, NP><<<grid, kThreads, 0, st>>>(a);
+  else norm_gate_kernel<T, true, false, VEC, LPG, NP><<<grid, kThreads, 0, st>>>(a);
   return launch_status();
+}
+
+// VEC = features per access.  16-byte accesses (8 features of a 16-bit type) need groups of a multiple
+// of 8 features and 16-byte aligned tensors; 16-bit tensors that have neither take 8-byte accesses.
+template <typename T, int VEC>
+int launch_vec(const NormArgs &a, bool bwd, cudaStream_t st) {
+  const int lanes = (a.e + VEC - 1) / VEC;
+  if (lanes <= 8) return launch_cfg<T, VEC, 8, 1>(a, bwd, st);
+  if (lanes <= 16) return launch_cfg<T, VEC, 16, 1>(a, bwd, st);
+  if (lanes <= 32) return launch_cfg<T, VEC, 32, 1>(a, bwd, st);
+  if (lanes <= 64) return launch_cfg<T, VEC, 32, 2>(a, bwd, st);
+  if constexpr (VEC == 4) return launch_cfg<T, VEC, 32, 4>(a, bwd, st);
+  return LA_ERR_UNSUPPORTED;
+}
+
+template <typename T>
+int launch_t(const NormArgs &a, bool bwd, cudaStream_t st) {
+  if constexpr (sizeof(T) == 2) {
+    const uintptr_t all = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.gate) |
+                          reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.d_out) |
+                          reinterpret_cast<uintptr_t>(a.dx) | reinterpret_cast<uintptr_t>(a.dgate);
+    if (a.e % 8 == 0 && (all & 15u) == 0) return launch_vec<T, 8>(a, bwd, st);
+  }
+  return launch_vec<T, 4>(a, bwd, st);
 }
 
 int dispatch(const NormArgs &a, int dtype, bool bwd, cudaStream_t st) {
@@ -255,7 +318,7 @@ int check(const void *x, int64_t rows, int64_t G, int64_t e, int dtype, int act,
   cudaGetLastError();
   if (x == nullptr) return LA_ERR_NULL_POINTER;
   if (rows <= 0 || G <= 0 || e <= 0) return LA_ERR_BAD_SHAPE;
-  if (e % 4 != 0 || e > 32 * kMaxPerLane || G > 65535) return LA_ERR_UNSUPPORTED;
+  if (e % 4 != 0 || e > kMaxFeatures || G > 65535) return LA_ERR_UNSUPPORTED;
   if (act < 0 || act > 3 || gate_pos < 0 || gate_pos > 1) return LA_ERR_UNSUPPORTED;
   if (!(dtype == LA_F32 || dtype == LA_BF16 || dtype == LA_F16)) return LA_ERR_UNSUPPORTED;
   return LA_OK;
