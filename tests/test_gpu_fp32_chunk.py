@@ -1,0 +1,65 @@
+"""GPU: the chunk-parallel fp32 forward (fp32 inputs, and 16-bit sequences shorter than a tensor-core tile)
+against the oracle in 64 bits, at the edges of its chunks, segments and feature tiles."""
+import pytest
+import torch
+
+from oracle import lightning_attn_oracle as orc
+from util import TOL_BF16, TOL_FP32, assert_close, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(b, n, h, d, e, dtype, seed=0):
+    gen = torch.Generator().manual_seed(seed + n + d)
+    q, k = (torch.randn(b, n, h, d, generator=gen).div(d ** 0.5).to(dtype) for _ in range(2))
+    v = torch.randn(b, n, h, e, generator=gen).to(dtype)
+    ld = torch.nn.functional.logsigmoid(torch.randn(b, n, h, generator=gen))
+    s0 = torch.randn(b, h, d, e, generator=gen)
+    return q, k, v, ld, s0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,e", [(4, 4), (32, 32), (36, 64), (64, 40), (128, 68), (128, 128)])
+@pytest.mark.parametrize("b,n,h", [(1, 16, 1), (2, 63, 2), (1, 64, 3), (2, 65, 2), (1, 127, 2), (3, 130, 120),
+                                   (1, 1000, 2)])
+def test_fp32_chunk_forward(b, n, h, d, e, dtype):
+    from xopes_b200 import lasd_recurrence_cuda, lightning_attn_func
+    if h == 120 and d != 36:
+        pytest.skip("more pairs than the launch aims at: one shape is enough")
+    q, k, v, ld, s0 = _inputs(b, n, h, d, e, dtype)
+    dev = [t.cuda() for t in (q, k, v, ld, s0)]
+    tol = TOL_FP32 if dtype == torch.float32 else TOL_BF16
+    for state in (None, s0):
+        o, sf = lightning_attn_func(*dev[:3], ld=dev[3], initial_state=None if state is None else dev[4],
+                                    decay_type="scalar")
+        ro, rs = orc.lasd_forward(q, k, v, ld, state, acc=torch.float64)
+        assert_close("o", ro.to(dtype) if dtype != torch.float32 else ro, o, tol)
+        assert_close("state", rs, sf, tol)
+        if dtype == torch.float32:  # no further from 64 bits than the token-by-token kernel (1e-7: ulp noise)
+            o2, s2 = lasd_recurrence_cuda(*dev[:4], initial_state=None if state is None else dev[4])
+            assert rel_l2(ro, o) <= rel_l2(ro, o2) + 1e-7 and rel_l2(rs, sf) <= rel_l2(rs, s2) + 1e-7
+
+
+def test_fp32_chunk_forward_decay_forms():
+    """Per-head and strided decays, pre-activations, decays of -inf (a reset) and of 0, and non-finite
+    values, which must reach the rows the recurrence reaches and no others."""
+    from xopes_b200 import lasd_recurrence_cuda, lightning_attn_func
+    q, k, v, ld, s0 = (t.cuda() for t in _inputs(2, 200, 3, 64, 64, torch.float32))
+    ld[:, 5] = float("-inf")
+    ld[:, 70:72] = float("-inf")
+    ld[:, 90:100] = 0.0
+    x = torch.randn(2, 200, 3, device="cuda")
+    forms = [(ld, None), (ld.permute(1, 2, 0).contiguous().permute(2, 0, 1), None),
+             (torch.tensor([-0.01, -3.0, -200.0], device="cuda"), None), (x, "logsigmoid")]
+    for dec, act in forms:
+        got = lightning_attn_func(q, k, v, ld=dec, initial_state=s0, decay_type="scalar", decay_activation=act)
+        ref = lasd_recurrence_cuda(q, k, v, ld=dec, initial_state=s0, decay_activation=act)
+        for name, r, g in zip(("o", "state"), ref, got):
+            assert_close(name, r, g, TOL_FP32)
+    v2 = v.clone()
+    v2[0, 37, 1, 3] = float("inf")
+    v2[1, 130, 0, 2] = float("nan")
+    got = lightning_attn_func(q, k, v2, ld=-x.abs(), initial_state=s0, decay_type="scalar")
+    ref = lasd_recurrence_cuda(q, k, v2, ld=-x.abs(), initial_state=s0)
+    for r, g in zip(ref, got):
+        assert torch.equal(torch.isfinite(r), torch.isfinite(g))

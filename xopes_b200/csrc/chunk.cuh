@@ -32,6 +32,17 @@ struct ChunkPass {
   int no_scratch = 0;  // 1: never take hand-off scratch from the library's pool (one CTA per pair)
 };
 
+// SM count of the current device (0 on error) and scratch in stream order from the pool the library
+// owns (free it with cudaFreeAsync on the same stream).
+int device_sms();
+int scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
+
+// Chunk-parallel scalar-decay forward in fp32 arithmetic (chunk_fp32.cu), without cu_seqlens; returns
+// LA_ERR_UNSUPPORTED for a call that belongs to the scan kernels.
+int launch_fp32_chunk_fwd(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb, int64_t ld_sn,
+                          int64_t ld_sh, const float *s0, void *o, float *s_fin, int B, int N, int H, int D, int E,
+                          int dtype, int ld_act, cudaStream_t st);
+
 bool chunk_supported(int64_t N, int64_t D, int64_t E, int dtype);
 // With more (sequence, head) pairs than SMs the launch runs one CTA per SM on an even split of
 // the chunk space; the running state of a pair cut by a split crosses through scratch taken from
