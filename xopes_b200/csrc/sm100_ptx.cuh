@@ -217,6 +217,13 @@ __host__ __device__ constexpr uint32_t instr_desc(uint32_t ab_format, uint32_t a
          ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
+// One lane of the (converged) warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.b32 %0, 1, 0, e;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                        uint32_t accumulate) {
