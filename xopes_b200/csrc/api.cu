@@ -453,7 +453,6 @@ int la_lavd_fwd(const void *q, const void *k, const void *v, const float *ldk, c
   if (path == 1) {
     int *unsafe = lavd_unsafe_ptr();
     if (unsafe == nullptr) return LA_ERR_CUDA;
-    if (cudaMemsetAsync(unsafe, 0, 2 * sizeof(int), st) != cudaSuccess) return LA_ERR_CUDA;
     LavdPass c;
     c.x = q; c.y = k; c.z = v; c.ldk = ldk; c.out = o; c.t0 = initial_state; c.tfinal = final_state;
     if (ldk == nullptr) {
@@ -465,9 +464,11 @@ int la_lavd_fwd(const void *q, const void *k, const void *v, const float *ldk, c
     c.B = s.B; c.N = s.N; c.H = s.H; c.M = s.M; c.cu = cu_seqlens; c.unsafe = unsafe;
     c.ld_act = (flags & LA_FLAG_LD_LOGSIGMOID) ? 1 : 0;
     c.ld16 = ld16;
+    c.skip = unsafe;
+    if ((rc = launch_lavd_sample(c.ldk, cu_seqlens, s.B, s.N, s.H, s.M, dtype, ld16, c.ld_act, unsafe, st)) != LA_OK) return rc;
     if ((rc = launch_lavd_pass(c, dtype, st)) != LA_OK) return rc;
     // the two-reference kernels run only if a chunk left the one-reference range ...
-    c.ref2 = 1; c.enable = unsafe; c.unsafe = unsafe + 1;
+    c.ref2 = 1; c.enable = unsafe; c.skip = nullptr; c.unsafe = unsafe + 1;
     if ((rc = launch_lavd_pass(c, dtype, st)) != LA_OK) return rc;
     enable = unsafe + 1;  // ... and the scan below only if one left theirs too
   }
@@ -509,10 +510,13 @@ int la_lavd_bwd(const void *q, const void *k, const void *v, const float *ldk, c
   if (path == 1) {
     int *unsafe = lavd_unsafe_ptr();
     if (unsafe == nullptr) return LA_ERR_CUDA;
-    if (cudaMemsetAsync(unsafe, 0, 2 * sizeof(int), st) != cudaSuccess) return LA_ERR_CUDA;
+    if ((rc = launch_lavd_sample(ldk != nullptr ? ldk : ldv, cu_seqlens, s.B, s.N, s.H, s.M, dtype, ld16,
+                                 (flags & LA_FLAG_LD_LOGSIGMOID) ? 1 : 0, unsafe, st)) != LA_OK)
+      return rc;
     LavdPass c;
     c.ld_act = (flags & LA_FLAG_LD_LOGSIGMOID) ? 1 : 0;
     c.ld16 = ld16;
+    c.skip = unsafe;
     c.ldk = ldk; c.B = s.B; c.N = s.N; c.H = s.H; c.M = s.M; c.cu = cu_seqlens; c.unsafe = unsafe;
     if (ldk == nullptr) {
       // Decay on the value features (ldv only): the four passes exchange roles with the key-decay
@@ -538,7 +542,7 @@ int la_lavd_bwd(const void *q, const void *k, const void *v, const float *ldk, c
       for (int level = 0; level < 2 && rc == LA_OK; ++level)
         for (int i = 0; i < 4 && rc == LA_OK; ++i) {
           LavdPass x = *order[i];
-          if (level == 1) { x.ref2 = 1; x.enable = unsafe; x.unsafe = unsafe + 1; }
+          if (level == 1) { x.ref2 = 1; x.enable = unsafe; x.skip = nullptr; x.unsafe = unsafe + 1; }
           rc = launch_lavd_pass(x, dtype, st);
         }
       if (rc != LA_OK) return rc;
@@ -571,6 +575,7 @@ int la_lavd_bwd(const void *q, const void *k, const void *v, const float *ldk, c
       LavdPass v2 = cv, q2 = cq, k2 = ck;
       v2.ref2 = q2.ref2 = k2.ref2 = 1;
       v2.enable = q2.enable = k2.enable = unsafe;
+      v2.skip = q2.skip = k2.skip = nullptr;
       v2.unsafe = q2.unsafe = k2.unsafe = unsafe + 1;
       q2.dld_add = k2.dld_add = 0;
       int r2 = launch_lavd_pass(v2, dtype, s_v);

@@ -77,7 +77,11 @@ struct LavdPass {
   int ld16 = 0;      // 1: ldk points to 16-bit values of the type of x, y, z
   int ref2 = 0;
   const int *enable = nullptr;  // optional device word: the launch does nothing while it reads 0
+  const int *skip = nullptr;    // optional device word: a CTA that finds it raised does nothing
 };
+// Clears unsafe[0..1] and raises unsafe[0] if a sample of the decays is out of the one-reference range.
+int launch_lavd_sample(const void *ldk, const int64_t *cu, int B, int N, int H, int M, int dtype, int ld16, int ld_act,
+                       int *unsafe, cudaStream_t st);
 bool lavd_chunk_supported(int64_t N, int64_t D, int64_t E, int dtype, bool has_ldk, bool has_ldv);
 int launch_lavd_pass(const LavdPass &p, int dtype, cudaStream_t stream);
 

@@ -32,7 +32,9 @@
 //                     Wb = P~bot[:, 64:128] Z'[64:128] + X (T e^{g-r3}), P~bot = P~ with rows 0..63
 //                     zeroed (a second 16-bit copy in the unused half of each batch of P).
 // The caller runs the one-reference kernels first; the REF2 kernels run only if those raised their
-// flag, and the scan kernels only if a 32-row quarter decays by more than 2^-96 (bf16).
+// flag, and the scan kernels only if a 32-row quarter decays by more than 2^-96 (bf16).  A one-block
+// sample of the decays (lavd_sample_kernel) raises the flag before the one-reference kernels where it
+// can, and these leave at once when they find it raised: their results would be thrown away.
 //
 // The factor e^{g-m} of the state update is not multiplied into the operand: it is owed to the
 // state (kept as T~ with T = T~ scaled per feature by the owed factor) and paid at the start of the
@@ -133,6 +135,7 @@ struct LavdArgs {
   int *status;
   int *unsafe;
   const int *enable;  // optional device word: the kernel does nothing while it reads 0
+  const int *skip;    // optional device word: a CTA that finds it raised does nothing
   int ld_act;         // 1: the decay tensor holds pre-activations x and the log decay is logsigmoid(x)
   int ld16;           // 1: the decay tensor has the 16-bit type of x, y, z (half the bytes per chunk)
 };
@@ -298,6 +301,8 @@ lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                  const LavdArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (a.enable != nullptr && *a.enable == 0) return;  // uniform over the grid
+  // another CTA may raise this word at any time: one verdict per CTA
+  if (a.skip != nullptr && __syncthreads_or(*static_cast<const volatile int *>(a.skip) != 0)) return;
   const uint32_t base = smem_u32(smem_raw);
   uint8_t *gbase = smem_raw;
   Small *sm = reinterpret_cast<Small *>(gbase + kOffSmall);
@@ -432,7 +437,9 @@ lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncwarp();
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ tensor-core issue
-    if (lane == 0) {
+    // the whole warp walks the loop and one elected lane issues, so that descriptors are uniform
+    // registers as the instruction wants them (see chunk_sm100.cu)
+    {
       const uint32_t idesc_kk = instr_desc(Fmt<T>::kAB, 0, 0, 128, 128);
       const uint32_t idesc_kk64 = instr_desc(Fmt<T>::kAB, 0, 0, 128, 64);
       const uint32_t idesc_kmn = instr_desc(Fmt<T>::kAB, 0, 1, 128, 128);
@@ -451,26 +458,29 @@ lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // N mode multiplies the rescaled X and Y; T mode the tiles as loaded
         if (!TMODE) mbar_wait(bar_r, par, abort_flag, a.status, kStR);
         tc_fence_after();
-        if (!TMODE && REF2) {
+        if (elect_one()) {
+          if (!TMODE && REF2) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
-            if (!rev) {  // P[:, 0:64] = X' R[0:64]^T ; P[:, 64:128] = R Y'[64:128]^T
-              mma_ss(tmem + kColP, d_xk + ko, d_rk + ko, idesc_kk64, ks > 0);
-              mma_ss(tmem + kColP + 64, d_rk + ko, d_yk + ko + kRow64, idesc_kk64, ks > 0);
-            } else {     // P[:, 0:64] = R Y'[0:64]^T ; P[:, 64:128] = X' R[64:128]^T
-              mma_ss(tmem + kColP, d_rk + ko, d_yk + ko, idesc_kk64, ks > 0);
-              mma_ss(tmem + kColP + 64, d_xk + ko, d_rk + ko + kRow64, idesc_kk64, ks > 0);
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
+              if (!rev) {  // P[:, 0:64] = X' R[0:64]^T ; P[:, 64:128] = R Y'[64:128]^T
+                mma_ss(tmem + kColP, d_xk + ko, d_rk + ko, idesc_kk64, ks > 0);
+                mma_ss(tmem + kColP + 64, d_rk + ko, d_yk + ko + kRow64, idesc_kk64, ks > 0);
+              } else {     // P[:, 0:64] = R Y'[0:64]^T ; P[:, 64:128] = X' R[64:128]^T
+                mma_ss(tmem + kColP, d_rk + ko, d_yk + ko, idesc_kk64, ks > 0);
+                mma_ss(tmem + kColP + 64, d_xk + ko, d_rk + ko + kRow64, idesc_kk64, ks > 0);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
+              mma_ss(tmem + kColP, d_xk + ko, d_yk + ko, idesc_kk, ks > 0);
             }
           }
-        } else {
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
-            mma_ss(tmem + kColP, d_xk + ko, d_yk + ko, idesc_kk, ks > 0);
-          }
+          mma_commit(bar_p);
         }
-        mma_commit(bar_p);
+        __syncwarp();
         mbar_wait(bar_d, par, abort_flag, a.status, kStD);
         if (TMODE) mbar_wait(bar_r, par, abort_flag, a.status, kStR);
         tc_fence_after();
@@ -478,61 +488,73 @@ lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // epilogue.  T mode with two references: it shares the accumulator whose output scale it
         // has (forward: Wa = columns W1, reverse: Wb = columns W2).
         const uint32_t col_xt = (TMODE && REF2 && !rev) ? kColW1 : kColW2;
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
-          mma_ss(tmem + col_xt, d_xk + ko, d_tb + (uint64_t)(ks * 128), idesc_kmn, ks > 0);
+          for (int ks = 0; ks < 8; ++ks) {
+            const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
+            mma_ss(tmem + col_xt, d_xk + ko, d_tb + (uint64_t)(ks * 128), idesc_kmn, ks > 0);
+          }
+          if (TMODE && REF2 && a.dld != nullptr) mma_commit(bar_x);
         }
+        __syncwarp();
         if (TMODE && REF2 && a.dld != nullptr) {   // low half of the split state copy (same tile, in turn)
-          mma_commit(bar_x);
           mbar_wait(bar_l, par, abort_flag, a.status, kStL);
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
-            mma_ss(tmem + col_xt, d_xk + ko, d_tb + (uint64_t)(ks * 128), idesc_kmn, 1);
-          }
-        }
-        if (TMODE && !REF2 && a.dld != nullptr) {  // low half of the split state copy (spare tile)
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
-            mma_ss(tmem + col_xt, d_xk + ko, d_fmn + (uint64_t)(ks * 128), idesc_kmn, 1);
-          }
-        }
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {  // state update Y^T Z (N mode: Y rescaled; T mode: Z rescaled)
-          uint64_t zb = d_zmn;
-          if (TMODE && REF2 && ((ks < 4) != rev)) zb = d_fmn;  // rows against the other reference
-          mma_ss(tmem + kColT, d_ymn + (uint64_t)(ks * 128), zb + (uint64_t)(ks * 128), idesc_mnmn, 1);
-        }
-        mbar_wait(bar_f, par, abort_flag, a.status, kStF);
-        tc_fence_after();
-        if (TMODE && REF2) {
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t pa = tmem + kColP + (ks >> 1) * 32 + (ks & 1) * 8;
-            const uint64_t zk = d_zmn + (uint64_t)(ks * 128), fk = d_fmn + (uint64_t)(ks * 128);
-            if (!rev) {
-              // Wa += P~[:, 0:64] Z'[0:64] (on top of X T) ; Wb = P~[:, 64:128] Z'[64:128]
-              if (ks < 4) mma_ts(tmem + kColW1, pa, zk, idesc_kmn, 1);
-              else mma_ts(tmem + kColW2, pa, zk, idesc_kmn, ks > 4);
-            } else {
-              // Wa = P~[:, 0:64] Z'[0:64] + P~[:, 64:128] F[64:128] ; Wb += P~bot[:, 64:128] Z'[64:128]
-              mma_ts(tmem + kColW1, pa, ks < 4 ? zk : fk, idesc_kmn, ks > 0);
-              if (ks >= 4) mma_ts(tmem + kColW2, pa + 16, zk, idesc_kmn, 1);
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
+              mma_ss(tmem + col_xt, d_xk + ko, d_tb + (uint64_t)(ks * 128), idesc_kmn, 1);
             }
           }
-        } else {
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks)  // W1 = P~ Z (T mode: Z is the rescaled tile)
-            mma_ts(tmem + kColW1, tmem + kColP + (ks >> 1) * 32 + (ks & 1) * 8, d_zmn + (uint64_t)(ks * 128),
-                   idesc_kmn, ks > 0);
+          __syncwarp();
         }
-        mma_commit(bar_w);
-        // Y and Z have no reader left once the products above are done: in N mode they go back
-        // to the producer for the next chunk's Y and Z, in T mode for its decay tile
-        mma_commit(TMODE ? empty_ck : empty_yz);
+        if (elect_one()) {
+          if (TMODE && !REF2 && a.dld != nullptr) {  // low half of the split state copy (spare tile)
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint64_t ko = (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2);
+              mma_ss(tmem + col_xt, d_xk + ko, d_fmn + (uint64_t)(ks * 128), idesc_kmn, 1);
+            }
+          }
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) {  // state update Y^T Z (N mode: Y rescaled; T mode: Z rescaled)
+            uint64_t zb = d_zmn;
+            if (TMODE && REF2 && ((ks < 4) != rev)) zb = d_fmn;  // rows against the other reference
+            mma_ss(tmem + kColT, d_ymn + (uint64_t)(ks * 128), zb + (uint64_t)(ks * 128), idesc_mnmn, 1);
+          }
+        }
+        __syncwarp();
+        mbar_wait(bar_f, par, abort_flag, a.status, kStF);
+        tc_fence_after();
+        if (elect_one()) {
+          if (TMODE && REF2) {
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint32_t pa = tmem + kColP + (ks >> 1) * 32 + (ks & 1) * 8;
+              const uint64_t zk = d_zmn + (uint64_t)(ks * 128), fk = d_fmn + (uint64_t)(ks * 128);
+              if (!rev) {
+                // Wa += P~[:, 0:64] Z'[0:64] (on top of X T) ; Wb = P~[:, 64:128] Z'[64:128]
+                if (ks < 4) mma_ts(tmem + kColW1, pa, zk, idesc_kmn, 1);
+                else mma_ts(tmem + kColW2, pa, zk, idesc_kmn, ks > 4);
+              } else {
+                // Wa = P~[:, 0:64] Z'[0:64] + P~[:, 64:128] F[64:128] ; Wb += P~bot[:, 64:128] Z'[64:128]
+                mma_ts(tmem + kColW1, pa, ks < 4 ? zk : fk, idesc_kmn, ks > 0);
+                if (ks >= 4) mma_ts(tmem + kColW2, pa + 16, zk, idesc_kmn, 1);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks)  // W1 = P~ Z (T mode: Z is the rescaled tile)
+              mma_ts(tmem + kColW1, tmem + kColP + (ks >> 1) * 32 + (ks & 1) * 8, d_zmn + (uint64_t)(ks * 128),
+                     idesc_kmn, ks > 0);
+          }
+          mma_commit(bar_w);
+          // Y and Z have no reader left once the products above are done: in N mode they go back
+          // to the producer for the next chunk's Y and Z, in T mode for its decay tile
+          mma_commit(TMODE ? empty_ck : empty_yz);
+        }
+        __syncwarp();
         mbar_wait(bar_w, par, abort_flag, a.status, kStW);
       }
     }
@@ -1084,6 +1106,36 @@ lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   }
 }
 
+// Clears the two range words of a call and raises the first one if a sample of the decays is out of
+// the one-reference kernels' range: the first 64 tokens of up to four (sequence, head) pairs, all
+// features, the same sums and the same limit as those kernels use.  Only a hint (they check every chunk
+// themselves): decays that are out of range everywhere, as unscaled logsigmoids are, are seen here for
+// a few microseconds instead of by a full set of passes (B 2, H 16, N 4096, forward + backward: 1.10 ms
+// before, 0.69 ms with the sample); decays that are in range pay those microseconds.
+template <typename LT>
+__global__ void __launch_bounds__(512) lavd_sample_kernel(const LT *ld, const long long *cu, int N, int H, int pairs,
+                                                           int ld_act, float limit, int *unsafe) {
+  const int f = threadIdx.x & 127, g = threadIdx.x >> 7;
+  const int p = pairs >= 4 ? (int)((long long)g * pairs / 4) : g;
+  bool bad = false;
+  if (p < pairs) {
+    const int seq = p / H, h = p - seq * H;
+    const long long t0 = cu != nullptr ? cu[seq] : 0, len = cu != nullptr ? cu[seq + 1] - t0 : N;
+    const LT *row = ld + (((cu != nullptr ? 0 : (long long)seq * N) + t0) * H + h) * kChunk + f;
+    if (len >= 64) {
+      float sum = 0.f;
+      float v[64];  // one memory round trip
+#pragma unroll
+      for (int r = 0; r < 64; ++r) v[r] = Cvt<LT>::to_f(row[(long long)r * H * kChunk]);
+#pragma unroll
+      for (int r = 0; r < 64; ++r) sum += ld_act ? log2_sigmoid(v[r]) : v[r] * kLog2e;
+      bad = -sum > limit;
+    }
+  }
+  const int any = __syncthreads_or(bad);
+  if (threadIdx.x < 2) unsafe[threadIdx.x] = threadIdx.x == 0 ? any : 0;
+}
+
 template <typename T, bool TMODE, bool REF2>
 int launch_t(const LavdPass &p, int dtype, cudaStream_t stream) {
   alignas(64) CUtensorMap mx, my, mz, ml, mo, md;
@@ -1107,6 +1159,7 @@ int launch_t(const LavdPass &p, int dtype, cudaStream_t stream) {
   a.status = status_word_ptr();
   a.unsafe = p.unsafe;
   a.enable = p.enable;
+  a.skip = p.skip;
   a.ld_act = p.ld_act;
   a.ld16 = p.ld16;
   if (a.status == nullptr || a.unsafe == nullptr) return LA_ERR_CUDA;
@@ -1119,6 +1172,20 @@ int launch_t(const LavdPass &p, int dtype, cudaStream_t stream) {
 }
 
 }  // namespace
+
+int launch_lavd_sample(const void *ldk, const int64_t *cu, int B, int N, int H, int M, int dtype, int ld16, int ld_act,
+                       int *unsafe, cudaStream_t st) {
+  const int pairs = (cu != nullptr ? M : B) * H;
+  const long long *c = reinterpret_cast<const long long *>(cu);
+  const float limit = dtype == LA_BF16 ? SafeBits<__nv_bfloat16>::value : SafeBits<__half>::value;
+  if (!ld16)
+    lavd_sample_kernel<float><<<1, 512, 0, st>>>(static_cast<const float *>(ldk), c, N, H, pairs, ld_act, limit, unsafe);
+  else if (dtype == LA_BF16)
+    lavd_sample_kernel<__nv_bfloat16><<<1, 512, 0, st>>>(static_cast<const __nv_bfloat16 *>(ldk), c, N, H, pairs, ld_act, limit, unsafe);
+  else
+    lavd_sample_kernel<__half><<<1, 512, 0, st>>>(static_cast<const __half *>(ldk), c, N, H, pairs, ld_act, limit, unsafe);
+  return launch_status();
+}
 
 bool lavd_chunk_supported(int64_t N, int64_t D, int64_t E, int dtype, bool has_ldk, bool has_ldv) {
   // exactly one decay: on the key features (ldk) or, by exchanging the roles of the passes, on the
