@@ -127,7 +127,7 @@ class LasdFunction(torch.autograd.Function):
             return o, sf
         o = torch.empty(b, n, h, e, dtype=q.dtype, device=q.device)
         sf = torch.empty(nb, h, d, e, dtype=torch.float32, device=q.device)
-        with torch.cuda.device(q.device):
+        with _lib.device_of(q):
             rc = lib.la_lasd_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
                                  _lib.ptr(s0), _lib.ptr(cu), _lib.ptr(o), _lib.ptr(sf),
                                  b, n, h, d, e, m, _lib.dtype_code(q), flags, _lib.stream_of(q))
@@ -178,7 +178,7 @@ class LasdFunction(torch.autograd.Function):
         if want_dld:
             ws_bytes = lib.la_lasd_bwd_workspace_bytes(b, n, h, d, e, m, 1)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-        with torch.cuda.device(q.device):
+        with _lib.device_of(q):
             rc = lib.la_lasd_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
                                  _lib.ptr(s0), _lib.ptr(do), _lib.ptr(dsf), _lib.ptr(cu),
                                  _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(dld),
@@ -256,7 +256,7 @@ def lasd_decode_step(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ld: torc
     ld32, (sb, _, sh) = _prep_ld(ld, b, 1, h)
     new_state = state if inplace else torch.empty_like(state)
     o = out if out is not None else torch.empty(b, 1, h, e, dtype=q.dtype, device=q.device)
-    with torch.cuda.device(q.device):
+    with _lib.device_of(q):
         rc = lib.la_decode_scalar(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sh,
                                   _lib.ptr(state), _lib.ptr(new_state), _lib.ptr(o), b, h, d, e,
                                   _lib.dtype_code(q), _lib.stream_of(q))

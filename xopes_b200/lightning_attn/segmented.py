@@ -191,7 +191,7 @@ def _incoming_states(lib, y, z, ld32, ld_strides, pl: _Plan, ext, reverse: bool,
     incoming = torch.empty(pl.nseg, h, d, e, dtype=torch.float32, device=dev)
     local = torch.empty(max(n_loc, 1), h, d, e, dtype=torch.float32, device=dev)
     gsum = torch.empty(max(n_loc, 1), h, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.device_of(y):
         if n_loc:
             rc = lib.la_lasd_state_pass(_lib.ptr(y), _lib.ptr(z), _lib.ptr(ld32), 0, sn, sh, _lib.ptr(fl["ranges"]),
                                         _lib.ptr(local), _lib.ptr(gsum), 1, t, h, d, e, n_loc,
@@ -220,7 +220,7 @@ def lasd_forward_segmented(q, k, v, ld32, ld_strides, initial_state, doc_bounds,
     o = torch.empty(1, t, h, e, dtype=q.dtype, device=dev)
     st = torch.empty(pl.nseg, h, d, e, dtype=torch.float32, device=dev)
     _, sn, sh = ld_strides
-    with torch.cuda.device(dev):
+    with _lib.device_of(q):
         rc = lib.la_lasd_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), 0, sn, sh, _lib.ptr(s_in),
                              _lib.ptr(pl.cu_dev), _lib.ptr(o), _lib.ptr(st), 1, t, h, d, e, pl.nseg,
                              _lib.dtype_code(q), (_lib.FLAG_REQUIRE_TENSOR if pl.cut else 0) | act, _lib.stream_of(q))
@@ -251,7 +251,7 @@ def lasd_forward_exchange_first(q, k, v, ld32, ld_strides, doc_bounds, cap, open
     local = torch.empty(max(n_loc, 1), h, d, e, dtype=torch.float32, device=dev)
     gsum = torch.empty(max(n_loc, 1), h, dtype=torch.float32, device=dev)
     s_end = None
-    with torch.cuda.device(dev):
+    with _lib.device_of(q):
         if n_loc:
             rc = lib.la_lasd_state_pass(_lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), 0, sn, sh, _lib.ptr(fl["ranges"]),
                                         _lib.ptr(local), _lib.ptr(gsum), 1, t, h, d, e, n_loc,
@@ -270,7 +270,7 @@ def lasd_forward_exchange_first(q, k, v, ld32, ld_strides, doc_bounds, cap, open
     incoming = torch.empty(pl.nseg, h, d, e, dtype=torch.float32, device=dev)
     o = torch.empty(1, t, h, e, dtype=q.dtype, device=dev)
     st = torch.empty(pl.nseg, h, d, e, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.device_of(q):
         rc = lib.la_lasd_fold_states(_lib.ptr(local), _lib.ptr(gsum), _lib.ptr(fl["table"]), _lib.ptr(fl["emit"]),
                                      _lib.ptr(ext), _lib.ptr(incoming), None, fl["nunits"], h, d, e, 0, stream)
         _lib.check(rc, "la_lasd_fold_states")
@@ -302,7 +302,7 @@ def lasd_backward_segmented(q, k, v, ld32, ld_strides, initial_state, do, dfinal
         ws_bytes = lib.la_lasd_bwd_workspace_bytes(1, t, h, d, e, pl.nseg, 1)
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     _, sn, sh = ld_strides
-    with torch.cuda.device(dev):
+    with _lib.device_of(q):
         rc = lib.la_lasd_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), 0, sn, sh, _lib.ptr(s_in),
                              _lib.ptr(do), _lib.ptr(ds_out), _lib.ptr(pl.cu_dev), _lib.ptr(dq), _lib.ptr(dk),
                              _lib.ptr(dv), _lib.ptr(dld), _lib.ptr(ds0), _lib.ptr(ws), ws_bytes, 1, t, h, d, e,
@@ -327,7 +327,7 @@ def _incoming_states_vec(lib, y, z, ldk, pl: _Plan, ext, reverse: bool, act: int
     incoming = torch.empty(pl.nseg, h, d, e, dtype=torch.float32, device=dev)
     local = torch.empty(max(n_loc, 1), h, d, e, dtype=torch.float32, device=dev)
     gsum = torch.empty(max(n_loc, 1), h, d, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.device_of(y):
         if n_loc:
             rc = lib.la_lavd_state_pass(_lib.ptr(y), _lib.ptr(z), _lib.ptr(ldk), _lib.ptr(fl["ranges"]),
                                         _lib.ptr(local), _lib.ptr(gsum), 1, t, h, d, e, n_loc,
@@ -372,7 +372,7 @@ def lavd_forward_segmented(q, k, v, ld, initial_state, doc_bounds, cap, flags, v
     o = torch.empty(1, t, h, e, dtype=q.dtype, device=dev)
     st = torch.empty(pl.nseg, h, d, e, dtype=torch.float32, device=dev)
     lk, lv = (None, ld) if value_decay else (ld, None)
-    with torch.cuda.device(dev):
+    with _lib.device_of(q):
         rc = lib.la_lavd_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(lk), _lib.ptr(lv), _lib.ptr(s_in),
                              _lib.ptr(pl.cu_dev), _lib.ptr(o), _lib.ptr(st), 1, t, h, d, e, pl.nseg,
                              _lib.dtype_code(q), flags, _lib.stream_of(q))
@@ -400,7 +400,7 @@ def lavd_backward_segmented(q, k, v, ld, initial_state, do, dfinal_state, doc_bo
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     lk, lv = (None, ld) if value_decay else (ld, None)
     dlk, dlv = (None, dld) if value_decay else (dld, None)
-    with torch.cuda.device(dev):
+    with _lib.device_of(q):
         rc = lib.la_lavd_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(lk), _lib.ptr(lv), _lib.ptr(s_in),
                              _lib.ptr(do), _lib.ptr(ds_out), _lib.ptr(pl.cu_dev), _lib.ptr(dq), _lib.ptr(dk),
                              _lib.ptr(dv), _lib.ptr(dlk), _lib.ptr(dlv), _lib.ptr(ds0), _lib.ptr(ws), ws_bytes,

@@ -112,7 +112,7 @@ def _cuda_correct(q, o, cum, s_in, t1):
     e = o.shape[-1]
     cum = cum.contiguous()
     s_in = s_in.contiguous()
-    with torch.cuda.device(q.device):
+    with _lib.device_of(q):
         rc = lib.la_seqpar_correct(_lib.ptr(q), _lib.ptr(o), _lib.ptr(cum), _lib.ptr(s_in), t1, n, h, d, e,
                                    _lib.dtype_code(q), _lib.stream_of(q))
     _lib.check(rc, "la_seqpar_correct")
@@ -146,7 +146,7 @@ def fold_incoming_state(gathered: torch.Tensor, rank: int, h: int, d: int, e: in
         lib = _lib.load()
         g = gathered.contiguous()
         s_in = torch.empty(h, d, e, dtype=torch.float32, device=g.device)
-        with torch.cuda.device(g.device):
+        with _lib.device_of(g):
             rc = lib.la_seqpar_fold(_lib.ptr(g), _lib.ptr(s_in), rank, h, d, e, _lib.stream_of(g))
         _lib.check(rc, "la_seqpar_fold")
         return s_in

@@ -96,7 +96,7 @@ class LavdFunction(torch.autograd.Function):
         ctx.seg = None
         o = torch.empty(b, n, h, e, dtype=q.dtype, device=q.device)
         sf = torch.empty(nb, h, d, e, dtype=torch.float32, device=q.device)
-        with torch.cuda.device(q.device):
+        with _lib.device_of(q):
             rc = lib.la_lavd_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(lk), _lib.ptr(lv),
                                  _lib.ptr(s0), _lib.ptr(cu), _lib.ptr(o), _lib.ptr(sf),
                                  b, n, h, d, e, m, _lib.dtype_code(q), flags, _lib.stream_of(q))
@@ -141,7 +141,7 @@ class LavdFunction(torch.autograd.Function):
         if dsf is not None:
             ws_bytes = lib.la_lavd_bwd_workspace_bytes(b, n, h, d, e, m)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-        with torch.cuda.device(q.device):
+        with _lib.device_of(q):
             rc = lib.la_lavd_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(lk), _lib.ptr(lv),
                                  _lib.ptr(s0), _lib.ptr(do), _lib.ptr(dsf), _lib.ptr(cu),
                                  _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(dldk),
@@ -258,7 +258,7 @@ def lavd_decode_step(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     lk, lv = _ld32(ldk), _ld32(ldv)
     new_state = state if inplace else torch.empty_like(state)
     o = out if out is not None else torch.empty(b, 1, h, e, dtype=q.dtype, device=q.device)
-    with torch.cuda.device(q.device):
+    with _lib.device_of(q):
         rc = lib.la_decode_vector(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(lk), _lib.ptr(lv),
                                   _lib.ptr(state), _lib.ptr(new_state), _lib.ptr(o), b, h, d, e,
                                   _lib.dtype_code(q), _lib.stream_of(q))

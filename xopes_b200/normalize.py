@@ -35,7 +35,7 @@ class NormalizeGateFunction(torch.autograd.Function):
         w32 = None if weight is None else weight.detach().float().contiguous()
         b32 = None if bias is None else bias.detach().float().contiguous()
         out = torch.empty_like(xc)
-        with torch.cuda.device(x.device):
+        with _lib.device_of(x):
             rc = lib.la_normalize_gate_fwd(_lib.ptr(xc), _lib.ptr(gc), _lib.ptr(w32), _lib.ptr(b32), _lib.ptr(out),
                                            rows, num_groups, e, _lib.dtype_code(xc), act, pos, c, eps,
                                            1 if use_mean else 0, _lib.stream_of(xc))
@@ -56,7 +56,7 @@ class NormalizeGateFunction(torch.autograd.Function):
         dg = None if gc is None else torch.empty_like(gc)
         dw = None if w32 is None else torch.zeros_like(w32)
         db = None if b32 is None else torch.zeros_like(b32)
-        with torch.cuda.device(xc.device):
+        with _lib.device_of(xc):
             rc = lib.la_normalize_gate_bwd(_lib.ptr(xc), _lib.ptr(gc), _lib.ptr(w32), _lib.ptr(b32), _lib.ptr(do),
                                            _lib.ptr(dx), _lib.ptr(dg), _lib.ptr(dw), _lib.ptr(db), rows, num_groups,
                                            e, _lib.dtype_code(xc), act, pos, c, eps, 1 if use_mean else 0,
