@@ -1129,10 +1129,12 @@ chunk_pass_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Lau
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-// wprefix[s] = sum over sequences before s of (chunks + kTaskUnits); one block
-__global__ void weight_prefix_kernel(const long long *cu, int M, long long *wprefix) {
+// wprefix[s] = sum over sequences before s of (chunks + kTaskUnits), and the hand-off flags to zero (a
+// memset in front of this cost a launch gap of 4 us per pass); one block
+__global__ void weight_prefix_kernel(const long long *cu, int M, long long *wprefix, int *flags, int nflags) {
   __shared__ long long part[1024];
   const int tid = threadIdx.x, per = (M + 1023) / 1024;
+  for (int i = tid; i < nflags; i += 1024) flags[i] = 0;
   const int lo = min(M, tid * per), hi = min(M, lo + per);
   long long sum = 0;
   for (int s = lo; s < hi; ++s) {
@@ -1287,12 +1289,14 @@ int launch_t(const ChunkPass &p, const ChunkPass *q, int dtype, cudaStream_t str
       sc.flags = reinterpret_cast<int *>(base);
       sc.handoff = reinterpret_cast<float *>(base + flag_bytes + prefix_bytes);
       sc.total = pairs * (((long long)p.N + kChunk - 1) / kChunk);
-      bool ok = cudaMemsetAsync(sc.flags, 0, flag_bytes, stream) == cudaSuccess;
-      if (ok && p.cu) {
+      bool ok;
+      if (p.cu) {
         long long *wp = reinterpret_cast<long long *>(base + flag_bytes);
         sc.wprefix = wp;
-        weight_prefix_kernel<<<1, 1024, 0, stream>>>(reinterpret_cast<const long long *>(p.cu), p.M, wp);
+        weight_prefix_kernel<<<1, 1024, 0, stream>>>(reinterpret_cast<const long long *>(p.cu), p.M, wp, sc.flags, (int)grid);
         ok = cudaGetLastError() == cudaSuccess;
+      } else {
+        ok = cudaMemsetAsync(sc.flags, 0, flag_bytes, stream) == cudaSuccess;
       }
       if (!ok) {
         cudaFreeAsync(scratch, stream);
