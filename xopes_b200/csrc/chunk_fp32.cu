@@ -7,7 +7,8 @@
 //   o_i = sum_{j <= i} (q_i . k_j) e^{c_i - c_j} v_j + e^{c_i} q_i S_in,    S_out = e^g S_in + sum_j e^{g - c_j} k_j v_j^T
 //
 // with c the cumulative log decay inside the chunk, held in double so that a difference of two large
-// sums keeps its relative accuracy; every e^{..} is one fp32 exponential of that difference.
+// sums keeps its relative accuracy; e^{c_i - c_j} is one fp32 exponential of that difference, the 64 factors of
+// a chunk's state update are rounded once from double.
 //
 // The sequence is cut into segments of whole chunks, one CTA per (segment, head) in each of three
 // launches: (1) every segment's own state from a zero start, (2) a fold that turns those into the
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(kThreads) seg_state_kernel(const Args a) {
     chunk_decays(a, b, h, t, rows, cs);
     __syncthreads();
     const double g = cs[kC - 1];
-    if (threadIdx.x < kC) wj[threadIdx.x] = expf((float)(g - cs[threadIdx.x]));
+    if (threadIdx.x < kC) wj[threadIdx.x] = (float)exp(g - cs[threadIdx.x]);
     __syncthreads();
     StateAcc<DT> acc;
     state_product<DT>(acc, ks, vs, wj, ty, tx);
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(kThreads) seg_out_kernel(const Args a) {
     load_tile<T, DT>(vs, static_cast<const T *>(a.v) + row * a.E, (int64_t)a.H * a.E, rows, a.E);
     chunk_decays(a, b, h, t, rows, cs);
     __syncthreads();
-    if (threadIdx.x < kC) wj[threadIdx.x] = expf((float)(cs[kC - 1] - cs[threadIdx.x]));
+    if (threadIdx.x < kC) wj[threadIdx.x] = (float)exp(cs[kC - 1] - cs[threadIdx.x]);
     // ---- P = Q K^T, rows 4 ty + r, columns tx + 16 s (the row pitch spreads these over the banks)
     {
       float p[4][4];
