@@ -258,11 +258,11 @@ class LasdStep:
 
 
 class LavdStep(LasdStep):
-    # forward: state-only pass, fold, chunk pass, and two launches that only run if the decay leaves
+    # forward: state-only pass, fold, decay sample, chunk pass, and two launches that only run if the decay leaves
     # the range of the one before (two-reference chunk pass, scan); backward: 1 state-only pass
-    # (reverse flow; the forward-flow states are kept from the forward), 1 fold, 3 chunk passes,
+    # (reverse flow; the forward-flow states are kept from the forward), 1 fold, 1 sample, 3 chunk passes,
     # 3 + 3 such conditional launches, 1 reverse cumulative sum
-    launches_per_step = 17
+    launches_per_step = 19
     main_launches = 4      # o, dq, dk, dv chunk passes
     kernel = "lavd_pass_kernel"
 

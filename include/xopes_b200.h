@@ -8,7 +8,7 @@
  * itself, once per device and on first need: a stream-ordered memory pool from which a tcgen05
  * launch that splits (sequence, head) pairs across CTAs takes its hand-off scratch
  * (cudaMallocFromPoolAsync / cudaFreeAsync on the caller's stream, about 10 MB per launch in
- * flight), and two non-blocking side streams with three events on which independent gradient
+ * flight) and the fp32 forward its segments' states (at most 2 x SMs + B H of D x E floats), and two non-blocking side streams with three events on which independent gradient
  * passes of one backward call run beside each other.  la_lasd_bwd_noalloc uses neither.  The
  * return value is LA_OK or a negative LA_ERR_* code; la_status_string() turns it into text.
  *
