@@ -63,3 +63,26 @@ def test_fp32_chunk_forward_decay_forms():
     ref = lasd_recurrence_cuda(q, k, v2, ld=-x.abs(), initial_state=s0)
     for r, g in zip(ref, got):
         assert torch.equal(torch.isfinite(r), torch.isfinite(g))
+
+
+def test_fp32_chunk_forward_in_a_graph():
+    """Captured with its scratch (several segments) and replayed on new inputs."""
+    from xopes_b200 import lightning_attn_func
+    q, k, v, ld, s0 = (t.cuda() for t in _inputs(1, 300, 2, 64, 64, torch.float32))
+
+    def call():
+        with torch.no_grad():
+            return lightning_attn_func(q, k, v, ld=ld, initial_state=s0, decay_type="scalar")
+
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o, sf = call()
+    for x in (q, k, v):
+        x.copy_(torch.randn_like(x))
+    for _ in range(2):
+        graph.replay()
+    ro, rs = call()
+    torch.cuda.synchronize()
+    assert torch.equal(o, ro) and torch.equal(sf, rs)
