@@ -98,3 +98,25 @@ def test_normalize_gate_lane_splits(e, offset, use_mean, pos):
     rg = torch.autograd.grad((ro * do.double()).sum(), [xr, gr, wr, br])
     for name, ref, got in zip(("o", "dx", "dgate", "dweight", "dbias"), (ro,) + rg, (o,) + g):
         assert_close(name, ref.float(), got.float(), TOL_BF16)
+
+
+@pytest.mark.parametrize("pos", ["pre", "post"])
+@pytest.mark.parametrize("rows", [1, 77])
+@pytest.mark.parametrize("e", [4, 64, 128, 136])
+def test_normalize_gate_zero_eps(e, rows, pos):
+    """eps = 0 with a row count that leaves lanes of a warp without a row (32 lanes hold 4, 2 or 1 rows here):
+    those lanes must add nothing to the gradients of weight and bias (0 / sqrt(0) does)."""
+    from xopes_b200.normalize import normalize_gate_fn
+    gen = torch.Generator().manual_seed(e + rows)
+    groups = 2
+    x, gate, do = (torch.randn(rows, groups * e, generator=gen).bfloat16().float() for _ in range(3))
+    w, b = 1 + 0.1 * torch.randn(groups * e, generator=gen), 0.1 * torch.randn(groups * e, generator=gen)
+    xc, gc = (t.bfloat16().cuda().requires_grad_() for t in (x, gate))
+    wc, bc = w.cuda().requires_grad_(), b.cuda().requires_grad_()
+    o = normalize_gate_fn(xc, wc, bc, gate=gc, gate_act="sigmoid", gate_pos=pos, c=e ** 0.5, eps=0.0, num_groups=groups)
+    g = torch.autograd.grad(o, [xc, gc, wc, bc], do.bfloat16().cuda())
+    xr, gr, wr, br = (t.clone().requires_grad_() for t in (x, gate, w, b))
+    ro = norc.normalize_gate(xr, wr, br, gr, "sigmoid", pos, e ** 0.5, 0.0, False, groups)
+    rg = torch.autograd.grad((ro * do.double()).sum(), [xr, gr, wr, br])
+    for name, ref, got in zip(("o", "dx", "dgate", "dweight", "dbias"), (ro,) + rg, (o,) + g):
+        assert_close(name, ref.float(), got.float(), TOL_BF16)

@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(kThreads, (ctas_per_sm<BWD, POST, VEC * NP>())
         z[j] = (p * LPG + gl) * VEC < e ? z[j] - mean : 0.f;  // zc (e is a multiple of VEC)
         s2 += z[j] * z[j];
       }
-    const float rsig = rsqrtf(lane_sum<LPG>(s2) + a.eps);
+    // a row past the end (s2 = 0) takes 1 for eps: at eps = 0 its 1 / sqrt(0) would reach dw as 0 * inf
+    const float rsig = rsqrtf(lane_sum<LPG>(s2) + (!BWD || RPW == 1 || live ? a.eps : 1.f));
     if (!BWD) {
       float o[N];
 #pragma unroll
