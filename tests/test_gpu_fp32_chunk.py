@@ -86,3 +86,19 @@ def test_fp32_chunk_forward_in_a_graph():
     ro, rs = call()
     torch.cuda.synchronize()
     assert torch.equal(o, ro) and torch.equal(sf, rs)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("row", [0, 1, 41, 42, 63, 64, 130, 199])
+def test_fp32_chunk_forward_non_finite_decay(row, bad):
+    """A decay that is not finite reaches its own token and those after it, as in the recurrence, and no token
+    before it: at even and odd rows, at the edges of a chunk."""
+    from xopes_b200 import lasd_recurrence_cuda, lightning_attn_func
+    q, k, v, ld, s0 = (t.cuda() for t in _inputs(2, 200, 3, 64, 64, torch.float32))
+    ld[1, row, 2] = bad
+    got = lightning_attn_func(q, k, v, ld=ld, initial_state=s0, decay_type="scalar")
+    ref = lasd_recurrence_cuda(q, k, v, ld=ld, initial_state=s0)
+    for r, g in zip(ref, got):
+        assert torch.equal(torch.isfinite(r), torch.isfinite(g))
+    if row:
+        assert_close("o before", ref[0][1, :row, 2], got[0][1, :row, 2], TOL_FP32)

@@ -91,13 +91,15 @@ __device__ __forceinline__ void chunk_decays(const Args &a, int64_t b, int h, in
       x[u] = l;
     }
     double s = x[0] + x[1];
-    const double own = s;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const double n = __shfl_up_sync(0xffffffffu, s, off);
       if (lane >= off) s += n;
     }
-    const double pre = s - own;
+    // the sum before this lane's rows is the lane before's, not s minus the own part: that would carry a decay
+    // that is not finite from an odd row to the even one before it
+    double pre = __shfl_up_sync(0xffffffffu, s, 1);
+    if (lane == 0) pre = 0.0;
     cs[2 * lane] = pre + x[0];
     cs[2 * lane + 1] = s;
   }
