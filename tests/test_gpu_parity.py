@@ -628,3 +628,21 @@ def test_lavd_narrow_heads_run_padded_on_the_tensor_path(shape, which, lens, act
     assert tuple(lc.grad.shape) == (b, n, h, f)
     assert_close("dld", rl, lc.grad, TOL_BF16)
     assert_close("dinitial_state", rs0, s0c.grad, TOL_BF16)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d", [40, 64, 72, 128])
+def test_lasd_narrow_head_infinite_value_in_the_decay_gradient(d, dtype):
+    """All values positive and one infinite v: q.dq of its token and of every later one is +inf, and so is the
+    decay gradient after it, whatever the head's width (features that only fill a tile have no share in it)."""
+    import xopes_b200 as xb
+    n, h, at = 256, 2, 200
+    gen = torch.Generator().manual_seed(d)
+    q, k, v, do = ((0.1 + torch.rand(1, n, h, d, generator=gen)).to(dtype) for _ in range(4))
+    v[0, at, 0, 3] = float("inf")
+    ld = torch.full((1, n, h), -0.01)
+    q, k, v, ld = (leaf(t) for t in (q, k, v, ld))
+    o, _ = xb.lasd_parallel_cuda(q, k, v, ld=ld)
+    dld, = torch.autograd.grad(o, [ld], do.to(DEV))
+    assert torch.equal(dld[0, at + 1:, 0], torch.full((n - at - 1,), float("inf"), device=DEV))
+    assert torch.isfinite(dld[0, :, 1]).all()

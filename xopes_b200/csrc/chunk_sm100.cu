@@ -1008,17 +1008,21 @@ chunk_pass_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Lau
                 const uint4 x4 = *piece;  // this row of the row-dot operand
                 const uint32_t xw[4] = {x4.x, x4.y, x4.z, x4.w};
                 uint32_t o[4];
+                // features past a narrow head's stay out of the sum: zero there, but the product can be inf * 0
+                const bool inside = F128 || 64 * wg + p8 * 8 < fz;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                   const float w0 = __uint_as_float(w[8 * pc + 2 * j]), w1 = __uint_as_float(w[8 * pc + 2 * j + 1]);
-                  const float2 f = Fmt<T>::unpack(xw[j]);
-                  rd = fmaf(f.x, w0, rd);
-                  rd = fmaf(f.y, w1, rd);
+                  if (inside) {
+                    const float2 f = Fmt<T>::unpack(xw[j]);
+                    rd = fmaf(f.x, w0, rd);
+                    rd = fmaf(f.y, w1, rd);
+                  }
                   o[j] = Fmt<T>::pack(w0, w1);
                 }
                 if (full_chunk) {
                   *piece = make_uint4(o[0], o[1], o[2], o[3]);
-                } else if (i < L && (F128 || 64 * wg + p8 * 8 < fz)) {
+                } else if (i < L && inside) {
                   reinterpret_cast<uint4 *>(static_cast<T *>(ap.out) + row_off + 64 * wg)[p8] = make_uint4(o[0], o[1], o[2], o[3]);
                 }
               }
