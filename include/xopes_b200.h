@@ -78,7 +78,7 @@ LA_API int la_lasd_path(int64_t N, int64_t D, int64_t E, int dtype, unsigned fla
 LA_API int la_device_status(void *stream, int *status_out);
 LA_API int la_device_status_clear(void *stream);
 
-/* Reads (and synchronises the stream for) what the last vector-decay call on this GPU left behind:
+/* Reads (and synchronises the stream for) what the last vector-decay call issued on this GPU left behind:
  * 0 = it ran on the one-reference tensor-core kernels, 1 = a chunk decayed too fast for those and
  * the two-reference tensor-core kernels reran it, 2 = those gave up too and the scan kernels reran
  * it.  No counterpart in the reference. */
@@ -172,8 +172,9 @@ LA_API int la_lasd_bwd_noalloc(const void *q, const void *k, const void *v, cons
  * decay by at most 2^-64 per feature (bf16; 2^-10 for fp16); if a chunk exceeds that, the
  * two-reference kernels rerun the call (safe while every 32-token quarter decays by at most 2^-96;
  * the reference's own benchmark decay logsigmoid(N(0,1)) is about 2^-37 per quarter); if a chunk
- * exceeds that too, the scan kernels rerun it.  The two flag words behind those decisions are per
- * GPU: vector-decay calls whose kernels overlap on one GPU must be serialised. */
+ * exceeds that too, the scan kernels rerun it.  The two flag words behind those decisions belong to
+ * the call (one of 4096 pairs per GPU, and as many again for calls under stream capture, whose graphs
+ * keep them), so calls on different streams and threads may overlap. */
 LA_API int la_lavd_path(int64_t N, int64_t D, int64_t E, int dtype, int has_ldk, int has_ldv,
                         unsigned flags);
 

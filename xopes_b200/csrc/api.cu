@@ -25,20 +25,43 @@ int *status_word_ptr() {
   return ptrs[dev];
 }
 
-// [0]: raised by the one-reference vector-decay chunk kernels when a chunk leaves their safe range
-// (the two-reference kernels then run); [1]: raised by those in turn (the scan kernels then run)
-__device__ int g_lavd_unsafe[2] = {0, 0};
+// Two words per vector-decay call.  [0]: raised by the one-reference vector-decay chunk kernels when a
+// chunk leaves their safe range (the two-reference kernels then run); [1]: raised by those in turn (the
+// scan kernels then run).  Every call takes a pair of its own, so calls that overlap on several streams
+// or threads decide for themselves; a pair comes round again after kLavdCalls calls.  A call that is
+// being captured keeps its pair for as long as the graph lives, so captures take theirs from a second set,
+// which calls outside a capture never use.
+constexpr unsigned kLavdCalls = 4096;
+__device__ int g_lavd_unsafe[2][kLavdCalls][2];
 
-static int *lavd_unsafe_ptr() {
-  static int *ptrs[64] = {nullptr};
+struct LavdWords {
+  std::mutex mu;
+  int *base = nullptr, *last = nullptr;  // last: the pair of the latest call
+  unsigned next[2] = {0, 0};
+};
+
+static LavdWords *lavd_words() {
+  static LavdWords words[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  if (ptrs[dev] == nullptr) {
+  LavdWords &w = words[dev];
+  std::lock_guard<std::mutex> lock(w.mu);
+  if (w.base == nullptr) {
     void *p = nullptr;
     if (cudaGetSymbolAddress(&p, g_lavd_unsafe) != cudaSuccess) return nullptr;
-    ptrs[dev] = static_cast<int *>(p);
+    w.base = w.last = static_cast<int *>(p);
   }
-  return ptrs[dev];
+  return &w;
+}
+
+static int *lavd_unsafe_take(cudaStream_t st) {
+  LavdWords *w = lavd_words();
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (w == nullptr || cudaStreamIsCapturing(st, &capturing) != cudaSuccess) return nullptr;
+  const int set = capturing != cudaStreamCaptureStatusNone ? 1 : 0;
+  std::lock_guard<std::mutex> lock(w->mu);
+  const unsigned i = w->next[set]++ % kLavdCalls;
+  return w->last = w->base + ((size_t)set * kLavdCalls + i) * 2;
 }
 
 namespace {
@@ -197,8 +220,13 @@ int la_device_status_clear(void *stream) {
 
 int la_debug_lavd_unsafe(void *stream, int *flag_out) {
   if (flag_out == nullptr) return LA_ERR_NULL_POINTER;
-  int *p = lavd_unsafe_ptr();
-  if (p == nullptr) return LA_ERR_CUDA;
+  LavdWords *words = lavd_words();
+  if (words == nullptr) return LA_ERR_CUDA;
+  const int *p = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(words->mu);
+    p = words->last;
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int w[2] = {0, 0};
   if (cudaMemcpyAsync(w, p, sizeof(w), cudaMemcpyDeviceToHost, st) != cudaSuccess) return LA_ERR_CUDA;
@@ -451,7 +479,7 @@ int la_lavd_fwd(const void *q, const void *k, const void *v, const float *ldk, c
   Seq s{(int)B, (int)N, (int)H, (int)D, (int)E, (int)M, cu_seqlens};
   const int *enable = nullptr;
   if (path == 1) {
-    int *unsafe = lavd_unsafe_ptr();
+    int *unsafe = lavd_unsafe_take(st);
     if (unsafe == nullptr) return LA_ERR_CUDA;
     LavdPass c;
     c.x = q; c.y = k; c.z = v; c.ldk = ldk; c.out = o; c.t0 = initial_state; c.tfinal = final_state;
@@ -508,7 +536,7 @@ int la_lavd_bwd(const void *q, const void *k, const void *v, const float *ldk, c
   if (path < 0) return path;
   const int *enable = nullptr;
   if (path == 1) {
-    int *unsafe = lavd_unsafe_ptr();
+    int *unsafe = lavd_unsafe_take(st);
     if (unsafe == nullptr) return LA_ERR_CUDA;
     if ((rc = launch_lavd_sample(ldk != nullptr ? ldk : ldv, cu_seqlens, s.B, s.N, s.H, s.M, dtype, ld16,
                                  (flags & LA_FLAG_LD_LOGSIGMOID) ? 1 : 0, unsafe, st)) != LA_OK)
