@@ -8,7 +8,8 @@
  * itself, once per device and on first need: a stream-ordered memory pool from which a tcgen05
  * launch that splits (sequence, head) pairs across CTAs takes its hand-off scratch
  * (cudaMallocFromPoolAsync / cudaFreeAsync on the caller's stream, about 10 MB per launch in
- * flight) and the fp32 forward its segments' states (at most 2 x SMs + B H of D x E floats), and two non-blocking side streams with three events on which independent gradient
+ * flight; under stream capture these become allocation nodes of the graph), and two non-blocking
+ * side streams with three events on which independent gradient
  * passes of one backward call run beside each other.  la_lasd_bwd_noalloc uses neither.  The
  * return value is LA_OK or a negative LA_ERR_* code; la_status_string() turns it into text.
  *
@@ -48,8 +49,8 @@ extern "C" {
 enum la_dtype { LA_F32 = 0, LA_BF16 = 1, LA_F16 = 2 };
 
 /* flags for the lasd/lavd entry points */
-#define LA_FLAG_FORCE_RECURRENCE 1u /* never take the tcgen05 chunk kernels                       */
-#define LA_FLAG_REQUIRE_TENSOR 2u   /* fail with LA_ERR_UNSUPPORTED instead of taking the scan     */
+#define LA_FLAG_FORCE_RECURRENCE 1u /* never take a chunk form: token by token                    */
+#define LA_FLAG_REQUIRE_TENSOR 2u   /* LA_ERR_UNSUPPORTED instead of the fp32 CUDA-core kernels    */
 /* The decay tensors (ld; ldk, ldv) hold PRE-ACTIVATIONS x and the log decay is logsigmoid(x), the
  * usual producer of these decays (benchmarks/lightning_attention/benchmark.py:308-317): the
  * kernels apply it where they read the decay, and the backward returns d/dx in dld / dldk / dldv
@@ -69,7 +70,8 @@ LA_API int la_abi_version(void);
 LA_API const char *la_status_string(int status);
 
 /* Which kernel family a call with these parameters runs: 1 = tcgen05/TMA chunk kernels,
- * 0 = fp32 CUDA-core scan kernels, negative = LA_ERR_*.  Pure host logic, no CUDA call. */
+ * 0 = fp32 CUDA-core kernels (token by token; the forward in chunks of 64 tokens where la_lasd_fwd_ws
+ * says so), negative = LA_ERR_*.  Pure host logic, no CUDA call. */
 LA_API int la_lasd_path(int64_t N, int64_t D, int64_t E, int dtype, unsigned flags);
 
 /* Device-side watchdog word.  The tcgen05 kernels bound every mbarrier wait; a wait that runs
@@ -115,6 +117,22 @@ LA_API int la_lasd_fwd(const void *q, const void *k, const void *v, const float 
                 const int64_t *cu_seqlens, void *o, float *final_state, int64_t B, int64_t N,
                 int64_t H, int64_t D, int64_t E, int64_t M, int dtype, unsigned flags,
                 void *stream);
+
+/* la_lasd_fwd with scratch from the caller, for the fp32 CUDA-core path (la_lasd_path 0).  Without
+ * cu_seqlens and LA_FLAG_FORCE_RECURRENCE, with D and E multiples of 4 up to 128, N >= 16 and aligned
+ * tensors (16 bytes for fp32 and the states, 8 for 16-bit) that path's forward runs in chunks of 64 tokens.
+ * Given la_lasd_fwd_workspace_bytes bytes (16-byte aligned) the chunks of few (sequence, head) pairs run
+ * side by side; with workspace NULL, as in la_lasd_fwd, each pair walks its chunks in turn, which takes no
+ * scratch and rounds differently.  Other calls need 0 bytes and ignore the workspace.  The kernels are
+ * chosen from the arguments alone, the same under stream capture, and nothing here allocates on this path.
+ * LA_ERR_WORKSPACE / LA_ERR_MISALIGNED: a workspace that is too small or not aligned. */
+LA_API int64_t la_lasd_fwd_workspace_bytes(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E,
+                                    int64_t M, int dtype, unsigned flags);
+LA_API int la_lasd_fwd_ws(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb,
+                int64_t ld_sn, int64_t ld_sh, const float *initial_state,
+                const int64_t *cu_seqlens, void *o, float *final_state, void *workspace,
+                int64_t workspace_bytes, int64_t B, int64_t N, int64_t H, int64_t D, int64_t E,
+                int64_t M, int dtype, unsigned flags, void *stream);
 
 /* Bytes of scratch la_lasd_bwd needs (0 when dld is not requested). */
 LA_API int64_t la_lasd_bwd_workspace_bytes(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E,

@@ -102,3 +102,64 @@ def test_fp32_chunk_forward_non_finite_decay(row, bad):
         assert torch.equal(torch.isfinite(r), torch.isfinite(g))
     if row:
         assert_close("o before", ref[0][1, :row, 2], got[0][1, :row, 2], TOL_FP32)
+
+
+def test_fp32_chunk_forward_first_used_in_a_graph():
+    """A process whose first call is under stream capture gets the results (to the bit) of a call outside."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from xopes_b200 import lightning_attn_func
+torch.manual_seed(0)
+q, k, v = (torch.randn(1, 300, 2, 64, device="cuda") for _ in range(3))
+ld = torch.nn.functional.logsigmoid(torch.randn(1, 300, 2, device="cuda"))
+call = lambda: lightning_attn_func(q, k, v, ld=ld, decay_type="scalar")
+with torch.no_grad():
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o, s = call()
+    graph.replay()
+    ro, rs = call()
+    torch.cuda.synchronize()
+assert torch.equal(o, ro) and torch.equal(s, rs), float((o - ro).abs().max())
+del graph
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("b,n,h,d", [(1, 1000, 2, 64), (2, 100, 3, 128), (1, 16, 1, 32)])
+def test_fp32_chunk_forward_workspace(b, n, h, d):
+    """Through the C ABI: with the workspace the library asks for, without one (the sequence in one piece), and
+    with one that is too small or not aligned (refused before anything is launched)."""
+    from xopes_b200 import _lib
+    lib = _lib.load()
+    q, k, v, ld, s0 = _inputs(b, n, h, d, d, torch.float32)
+    dev = [t.cuda() for t in (q, k, v, ld, s0)]
+    o, sf = torch.empty_like(dev[2]), torch.empty_like(dev[4])
+    need = lib.la_lasd_fwd_workspace_bytes(b, n, h, d, d, 0, _lib.LA_F32, 0)
+    assert (need > 0) == (n > 64)
+    ws = torch.empty(need + 16, dtype=torch.uint8, device="cuda")
+
+    def call(at, nbytes):
+        o.fill_(float("nan"))
+        rc = lib.la_lasd_fwd_ws(*(t.data_ptr() for t in dev[:4]), *dev[3].stride(), dev[4].data_ptr(), None, o.data_ptr(),
+                                sf.data_ptr(), at, nbytes, b, n, h, d, d, 0, _lib.LA_F32, 0,
+                                torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return rc
+
+    ro, rs = orc.lasd_forward(q, k, v, ld, s0, acc=torch.float64)
+    for at, nbytes in ((ws.data_ptr(), need), (None, 0)):
+        assert call(at, nbytes) == 0
+        assert_close("o", ro, o, TOL_FP32)
+        assert_close("state", rs, sf, TOL_FP32)
+    if need:
+        assert call(ws.data_ptr(), need - 1) == -7 and call(ws.data_ptr() + 8, need) == -6
+        assert torch.isnan(o).all()
+    for case in ((b, n, h, d, d, 0, _lib.LA_F32, _lib.FLAG_FORCE_RECURRENCE), (1, n, h, d, d, 1, _lib.LA_F32, 0),
+                 (b, 256, h, d, d, 0, _lib.LA_BF16, 0), (b, 15, h, d, d, 0, _lib.LA_F32, 0), (b, n, h, d, 132, 0, _lib.LA_F32, 0)):
+        assert lib.la_lasd_fwd_workspace_bytes(*case) == 0

@@ -34,6 +34,9 @@ SIGNATURES = {
     "la_debug_umma_probe": (_i32, [_i32, _vp, _vp, _vp, _i32, _vp]),
     "la_lasd_fwd": (_i32, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp,
                            _i64, _i64, _i64, _i64, _i64, _i64, _i32, _u32, _vp]),
+    "la_lasd_fwd_workspace_bytes": (_i64, [_i64, _i64, _i64, _i64, _i64, _i64, _i32, _u32]),
+    "la_lasd_fwd_ws": (_i32, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _i64,
+                              _i64, _i64, _i64, _i64, _i64, _i64, _i32, _u32, _vp]),
     "la_lasd_bwd_workspace_bytes": (_i64, [_i64, _i64, _i64, _i64, _i64, _i64, _i32]),
     "la_lasd_bwd": (_i32, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                            _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i32, _u32,

@@ -526,48 +526,65 @@ int launch_t(Args &a, cudaStream_t st) {
 
 }  // namespace
 
-// LA_ERR_UNSUPPORTED: the call is one for the scan kernels.
+namespace {
+
+// Shapes the chunk form takes: four features per access; below 16 tokens the scan's few steps are as quick
+// as these launches.
+bool takes(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E) {
+  return D <= 128 && E <= 128 && D % 4 == 0 && E % 4 == 0 && N >= 16 && B * H <= 65535;
+}
+
+// Chunks per segment: as many segments as keep about two CTAs per SM (the states of the segments are then
+// at most 2 x SMs + B H of D x E floats, whatever N is).
+int chunks_per_segment(int64_t B, int64_t N, int64_t H) {
+  const int64_t chunks = (N + kC - 1) / kC, pairs = B * H, sms = device_sms();
+  int64_t parts = (2 * sms + pairs - 1) / pairs;
+  if (parts < 1) parts = 1;
+  if (parts > chunks) parts = chunks;
+  return (int)((chunks + parts - 1) / parts);
+}
+
+}  // namespace
+
+int64_t fp32_chunk_fwd_workspace(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E) {
+  if (!takes(B, N, H, D, E)) return 0;
+  const int64_t tokens = (int64_t)chunks_per_segment(B, N, H) * kC, nseg = (N + tokens - 1) / tokens;
+  return nseg > 1 ? B * H * nseg * (D * E + 1) * (int64_t)sizeof(float) : 0;
+}
+
+// LA_ERR_UNSUPPORTED: the call is one for the scan kernels.  Without a workspace the whole sequence is one
+// segment: no scratch, one launch.
 int launch_fp32_chunk_fwd(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb, int64_t ld_sn,
-                          int64_t ld_sh, const float *s0, void *o, float *s_fin, int B, int N, int H, int D, int E,
-                          int dtype, int ld_act, cudaStream_t st) {
-  // Four features per access, one 16-byte aligned row start per tensor; below 16 tokens the scan's
-  // few steps are as quick as these launches.
-  if (D > 128 || E > 128 || D % 4 != 0 || E % 4 != 0 || N < 16 || (int64_t)B * H > 65535) return LA_ERR_UNSUPPORTED;
+                          int64_t ld_sh, const float *s0, void *o, float *s_fin, void *workspace, int64_t workspace_bytes,
+                          int B, int N, int H, int D, int E, int dtype, int ld_act, cudaStream_t st) {
+  if (!takes(B, N, H, D, E)) return LA_ERR_UNSUPPORTED;
+  // one 16-byte aligned row start per tensor
   const uintptr_t rows = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                          reinterpret_cast<uintptr_t>(o);
   const uintptr_t states = reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(s_fin);
   if ((rows & (dtype == LA_F32 ? 15u : 7u)) != 0 || (states & 15u) != 0) return LA_ERR_UNSUPPORTED;
-  const int sms = device_sms();
-  if (sms <= 0) return LA_ERR_CUDA;
+  const int64_t need = fp32_chunk_fwd_workspace(B, N, H, D, E);
+  const bool cut = need > 0 && workspace != nullptr;
+  if (cut && workspace_bytes < need) return LA_ERR_WORKSPACE;
+  if (cut && (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return LA_ERR_MISALIGNED;
+  const int chunks = (N + kC - 1) / kC;
   Args a = {};
   a.q = q; a.k = k; a.v = v; a.ld = ld; a.ld_sb = ld_sb; a.ld_sn = ld_sn; a.ld_sh = ld_sh;
   a.s0 = s0; a.s_fin = s_fin; a.o = o;
   a.B = B; a.N = N; a.H = H; a.D = D; a.E = E; a.ld_act = ld_act;
-  // As many segments as keep about two CTAs per SM (the states of the segments are then at most
-  // 2 x SMs + B H of D x E floats, whatever N is).
-  const int chunks = (N + kC - 1) / kC;
-  const int64_t pairs = (int64_t)B * H;
-  int64_t parts = (2 * (int64_t)sms + pairs - 1) / pairs;
-  if (parts > chunks) parts = chunks;
-  const int per = (int)((chunks + parts - 1) / parts);
+  const int per = cut ? chunks_per_segment(B, N, H) : chunks;
   a.nseg = (chunks + per - 1) / per;
   a.seg_tokens = per * kC;
-  void *scratch = nullptr;
-  if (a.nseg > 1) {
-    const size_t state_bytes = (size_t)pairs * a.nseg * D * E * sizeof(float);
-    if (scratch_alloc(&scratch, state_bytes + (size_t)pairs * a.nseg * sizeof(float), st) != LA_OK)
-      return LA_ERR_UNSUPPORTED;
-    a.seg_state = static_cast<float *>(scratch);
-    a.seg_decay = reinterpret_cast<float *>(static_cast<char *>(scratch) + state_bytes);
+  if (cut) {
+    a.seg_state = static_cast<float *>(workspace);
+    a.seg_decay = a.seg_state + (int64_t)B * H * a.nseg * D * E;
   }
-  int rc = LA_ERR_UNSUPPORTED;
   switch (dtype) {
-    case LA_F32: rc = launch_t<float>(a, st); break;
-    case LA_BF16: rc = launch_t<__nv_bfloat16>(a, st); break;
-    case LA_F16: rc = launch_t<__half>(a, st); break;
+    case LA_F32: return launch_t<float>(a, st);
+    case LA_BF16: return launch_t<__nv_bfloat16>(a, st);
+    case LA_F16: return launch_t<__half>(a, st);
   }
-  if (scratch != nullptr && cudaFreeAsync(scratch, st) != cudaSuccess && rc == LA_OK) rc = LA_ERR_CUDA;
-  return rc;
+  return LA_ERR_UNSUPPORTED;
 }
 
 }  // namespace la

@@ -127,10 +127,15 @@ class LasdFunction(torch.autograd.Function):
             return o, sf
         o = torch.empty(b, n, h, e, dtype=q.dtype, device=q.device)
         sf = torch.empty(nb, h, d, e, dtype=torch.float32, device=q.device)
+        ws, ws_bytes = None, 0
         with _lib.device_of(q):
-            rc = lib.la_lasd_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
-                                 _lib.ptr(s0), _lib.ptr(cu), _lib.ptr(o), _lib.ptr(sf),
-                                 b, n, h, d, e, m, _lib.dtype_code(q), flags, _lib.stream_of(q))
+            if n < 128 or q.dtype == torch.float32:  # the fp32 CUDA-core path: states of its segments
+                ws_bytes = lib.la_lasd_fwd_workspace_bytes(b, n, h, d, e, m, _lib.dtype_code(q), flags)
+                if ws_bytes:
+                    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+            rc = lib.la_lasd_fwd_ws(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
+                                    _lib.ptr(s0), _lib.ptr(cu), _lib.ptr(o), _lib.ptr(sf), _lib.ptr(ws), ws_bytes,
+                                    b, n, h, d, e, m, _lib.dtype_code(q), flags, _lib.stream_of(q))
         _lib.check(rc, "la_lasd_fwd")
         ctx.save_for_backward(q, k, v, ld, s0, cu, None)
         ctx.flags = flags
