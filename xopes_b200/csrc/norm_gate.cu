@@ -128,14 +128,17 @@ __global__ void __launch_bounds__(kThreads, (ctas_per_sm<BWD, POST, VEC * NP>())
   R rx[NP], rg[NP], rd[NP];
   const R zero = {};
   auto fetch = [&](long long r) {
-    const long long off = r * stride + (long long)g * e;
+    // past the end: the last row again, with do = 0, so that such a lane adds 0 times a value of that row to the
+    // gradient sums (x = 0 in its place would make that 0 * inf at eps = 0)
+    const bool in = r < a.rows;
+    const long long off = (in ? r : a.rows - 1) * stride + (long long)g * e;
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int f = (p * LPG + gl) * VEC;
-      const bool on = r < a.rows && f < e;
+      const bool on = f < e;
       rx[p] = on ? *reinterpret_cast<const R *>(xp + off + f) : zero;
       rg[p] = (on && has_gate) ? *reinterpret_cast<const R *>(gp + off + f) : zero;
-      if (BWD) rd[p] = on ? *reinterpret_cast<const R *>(dp + off + f) : zero;
+      if (BWD) rd[p] = (on && in) ? *reinterpret_cast<const R *>(dp + off + f) : zero;
     }
   };
   const long long first = ((long long)blockIdx.x * kWarps + warp) * RPW;  // uniform over the warp
@@ -173,8 +176,7 @@ __global__ void __launch_bounds__(kThreads, (ctas_per_sm<BWD, POST, VEC * NP>())
         z[j] = (p * LPG + gl) * VEC < e ? z[j] - mean : 0.f;  // zc (e is a multiple of VEC)
         s2 += z[j] * z[j];
       }
-    // a row past the end (s2 = 0) takes 1 for eps: at eps = 0 its 1 / sqrt(0) would reach dw as 0 * inf
-    const float rsig = rsqrtf(lane_sum<LPG>(s2) + (!BWD || RPW == 1 || live ? a.eps : 1.f));
+    const float rsig = rsqrtf(lane_sum<LPG>(s2) + a.eps);
     if (!BWD) {
       float o[N];
 #pragma unroll
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, (ctas_per_sm<BWD, POST, VEC * NP>())
         const float y = a.c * xh * w[j] + b[j];
         const float dy = post ? d_o[j] * act[j] : d_o[j];
         dga[j] = post ? d_o[j] * y : 0.f;                // d loss / d act(gate), post-gate part
-        dw[j] += dy * a.c * xh;                          // rows past the end add zero: do reads as zero there
+        dw[j] += dy * a.c * xh;                          // rows past the end add zero (fetch)
         db[j] += dy;
         dxh[j] = dy * w[j] * a.c;
         dot += dxh[j] * xh;
