@@ -120,7 +120,8 @@ LA_API int la_lasd_fwd(const void *q, const void *k, const void *v, const float 
 
 /* la_lasd_fwd with scratch from the caller, for the fp32 CUDA-core path (la_lasd_path 0).  Without
  * cu_seqlens and LA_FLAG_FORCE_RECURRENCE, with D and E multiples of 4 up to 128, N >= 16 and aligned
- * tensors (16 bytes for fp32 and the states, 8 for 16-bit) that path's forward runs in chunks of 64 tokens.
+ * tensors (16 bytes for fp32 and the states, 8 for 16-bit) that path's forward runs in chunks of 64 tokens
+ * where sizes and the SM count say that this is quicker than token by token.
  * Given la_lasd_fwd_workspace_bytes bytes (16-byte aligned) the chunks of few (sequence, head) pairs run
  * side by side; with workspace NULL, as in la_lasd_fwd, each pair walks its chunks in turn, which takes no
  * scratch and rounds differently.  Other calls need 0 bytes and ignore the workspace.  The kernels are

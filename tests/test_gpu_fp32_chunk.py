@@ -163,3 +163,27 @@ def test_fp32_chunk_forward_workspace(b, n, h, d):
     for case in ((b, n, h, d, d, 0, _lib.LA_F32, _lib.FLAG_FORCE_RECURRENCE), (1, n, h, d, d, 1, _lib.LA_F32, 0),
                  (b, 256, h, d, d, 0, _lib.LA_BF16, 0), (b, 15, h, d, d, 0, _lib.LA_F32, 0), (b, n, h, d, 132, 0, _lib.LA_F32, 0)):
         assert lib.la_lasd_fwd_workspace_bytes(*case) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("b,h,n,d,chunks", [
+    (16, 16, 16, 128, False), (64, 16, 20, 64, False), (25, 12, 129, 32, False), (4, 50, 65, 32, False),  # many pairs
+    (25, 12, 130, 128, True), (20, 15, 64, 64, True), (1, 16, 100, 32, True), (10, 15, 127, 128, True),
+    (1, 2, 16, 128, False), (1, 2, 24, 128, True)])  # few tokens
+def test_fp32_chunk_forward_or_scan(b, h, n, d, chunks, dtype):
+    """Which form a call takes follows its sizes: where the scan is quicker it runs (equal to the bit), else the
+    chunk form; both agree with the oracle."""
+    from xopes_b200 import lasd_recurrence_cuda, lightning_attn_func
+    if dtype != torch.float32 and n >= 128:
+        pytest.skip("tensor-core path")
+    q, k, v, ld, s0 = _inputs(b, n, h, d, d, dtype)
+    dev = [t.cuda() for t in (q, k, v, ld, s0)]
+    o, sf = lightning_attn_func(*dev[:3], ld=dev[3], initial_state=dev[4], decay_type="scalar")
+    o2, s2 = lasd_recurrence_cuda(*dev[:4], initial_state=dev[4])
+    assert (torch.equal(o, o2) and torch.equal(sf, s2)) != chunks
+    tol = TOL_FP32 if dtype == torch.float32 else TOL_BF16
+    assert_close("o", o2, o, tol)
+    assert_close("state", s2, sf, tol)
+    ro, rs = orc.lasd_forward(q[:1, :, :2], k[:1, :, :2], v[:1, :, :2], ld[:1, :, :2], s0[:1, :2], acc=torch.float64)
+    assert_close("o against the oracle", ro.to(dtype) if dtype != torch.float32 else ro, o[:1, :, :2], tol)
+    assert_close("state against the oracle", rs, sf[:1, :2], tol)

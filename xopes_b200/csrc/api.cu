@@ -290,10 +290,10 @@ int la_lasd_fwd_ws(const void *q, const void *k, const void *v, const float *ld,
     return launch_chunk_pass(c, dtype, st);
   }
   const int ld_act = (flags & LA_FLAG_LD_LOGSIGMOID) ? 1 : 0;
-  // fp32 inputs and 16-bit sequences shorter than a tensor-core tile: the same arithmetic by chunks
-  // (B 2, H 8, N 512, D 64, fp32: 24 us against 394 us by tokens).  What it does not take (packed streams,
-  // odd or large head dimensions, a handful of tokens) and an explicit request for the recurrence
-  // run token by token.
+  // fp32 inputs and 16-bit sequences shorter than a tensor-core tile: the same arithmetic by chunks where that
+  // is quicker (B 2, H 8, N 512, D 64, fp32: 24 us against 394 us by tokens; the rule is in chunk_fp32.cu).
+  // What that does not take (packed streams, odd or large head dimensions, a handful of tokens) and an
+  // explicit request for the recurrence run token by token.
   if (!(flags & LA_FLAG_FORCE_RECURRENCE) && cu_seqlens == nullptr) {
     rc = launch_fp32_chunk_fwd(q, k, v, ld, ld_sb, ld_sn, ld_sh, initial_state, o, final_state, workspace,
                                workspace_bytes, s.B, s.N, s.H, s.D, s.E, dtype, ld_act, st);

@@ -524,32 +524,59 @@ int launch_t(Args &a, cudaStream_t st) {
   return launch_dt<T, 128>(a, st);
 }
 
-}  // namespace
+// How a call is cut: chunks per segment and segments per sequence; per = 0: a call for the scan.
+struct Plan {
+  int per, nseg;
+};
 
-namespace {
-
-// Shapes the chunk form takes: four features per access; below 16 tokens the scan's few steps are as quick
-// as these launches.
-bool takes(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E) {
-  return D <= 128 && E <= 128 && D % 4 == 0 && E % 4 == 0 && N >= 16 && B * H <= 65535;
+// The shapes the chunk form takes (four features per access) and, of those, the ones it is quicker for.
+// Below 16 tokens the scan's few steps are as quick as these launches.
+//
+// A CTA works on all 64 rows of a chunk and on a square tile of features however few of them there are, and
+// holds 50, 86 or 185 KB of shared memory, so its time goes by chunks and by CTAs per SM.  The scan's goes by
+// the tokens: a step's latency while the GPU has room (its CTAs grow once there are two per SM), then its
+// arithmetic on the padded state.  The constants are fitted to 1193 calls (fp32 and bf16; 4 to 128 features, D
+// and E equal or not; 16 to 2048 tokens; 1 to 8192 pairs), e.g., in us, chunk form / scan:
+//   128 features   64 tokens, 16 pairs 31 / 95, 8192 pairs 1697 / 3531;  16 tokens, 8192 pairs 1553 / 1025
+//    32 features   64 tokens, 16 pairs 13 / 37, 8192 pairs 452 / 282;  2048 tokens, 16 pairs 46 / 1081
+// Among those the choice is never slower than the scan by more than 2 us, and where it stays with the scan that
+// costs at most 1.24 times the chunk form's time (32 tokens of 192 pairs of 16 features, 21 us).
+Plan plan_of(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E, bool scratch) {
+  if (D > 128 || E > 128 || D % 4 != 0 || E % 4 != 0 || N < 16 || B * H > 65535) return {0, 0};
+  const int64_t pairs = B * H, chunks = (N + kC - 1) / kC, sms = device_sms() > 0 ? device_sms() : 1;
+  // with scratch, as many segments as keep about two CTAs per SM (the states of the segments are then at most
+  // 2 x SMs + B H of D x E floats, whatever N is)
+  int64_t parts = scratch ? (2 * sms + pairs - 1) / pairs : 1;
+  if (parts > chunks) parts = chunks;
+  const int64_t per = (chunks + parts - 1) / parts, nseg = (chunks + per - 1) / per;
+  const int tile = D > 64 || E > 64 ? 2 : (D > 32 || E > 32 ? 1 : 0), cols = D > 64 ? 2 : (D > 32 ? 1 : 0);
+  static const double kChunkUs[3] = {7.8, 11.8, 27.5}, kStartUs[3] = {5.0, 4.0, 1.5};
+  const double ctas_per_sm = (double)((pairs * nseg + sms - 1) / sms);
+  double chunk_us = kStartUs[tile] + kChunkUs[tile] * ctas_per_sm * per;
+  if (nseg > 1) chunk_us = kStartUs[tile] + 6.0 + 1.2 * kChunkUs[tile] * ctas_per_sm * per;  // three launches
+  // a scan step's latency: up to 32 pairs, fewer pairs than SMs, fewer than two per SM, more (with few rows
+  // the CTAs of 128 columns stay small)
+  static const double kStepUs[4][3] = {{0.53, 0.77, 1.35}, {0.47, 0.58, 0.9}, {0.45, 0.56, 1.5}, {0.47, 0.66, 1.6}};
+  static const double kElementUs[3] = {5.0e-7, 3.45e-7, 3.9e-7};  // per state element of a pair and token
+  int level = pairs <= 32 ? 0 : (pairs < sms ? 1 : (pairs < 2 * sms ? 2 : 3));
+  if (cols == 2 && level > 1 && (E <= 32 || (E <= 64 && level == 2))) level = 1;
+  int64_t rows = 8;
+  while (rows < E) rows *= 2;
+  const double work_us = kElementUs[cols] * (double)(32 << cols) * (double)rows * (double)pairs * 148.0 / (double)sms;
+  const double step_us = kStepUs[level][cols];
+  const double scan_us = 4.5 + (double)N * (work_us > step_us ? work_us : step_us);
+  if (chunk_us > scan_us) return {0, 0};
+  return {(int)per, (int)nseg};
 }
 
-// Chunks per segment: as many segments as keep about two CTAs per SM (the states of the segments are then
-// at most 2 x SMs + B H of D x E floats, whatever N is).
-int chunks_per_segment(int64_t B, int64_t N, int64_t H) {
-  const int64_t chunks = (N + kC - 1) / kC, pairs = B * H, sms = device_sms();
-  int64_t parts = (2 * sms + pairs - 1) / pairs;
-  if (parts < 1) parts = 1;
-  if (parts > chunks) parts = chunks;
-  return (int)((chunks + parts - 1) / parts);
+int64_t plan_bytes(const Plan &p, int64_t pairs, int64_t D, int64_t E) {
+  return p.nseg > 1 ? pairs * p.nseg * (D * E + 1) * (int64_t)sizeof(float) : 0;
 }
 
 }  // namespace
 
 int64_t fp32_chunk_fwd_workspace(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E) {
-  if (!takes(B, N, H, D, E)) return 0;
-  const int64_t tokens = (int64_t)chunks_per_segment(B, N, H) * kC, nseg = (N + tokens - 1) / tokens;
-  return nseg > 1 ? B * H * nseg * (D * E + 1) * (int64_t)sizeof(float) : 0;
+  return plan_bytes(plan_of(B, N, H, D, E, true), B * H, D, E);
 }
 
 // LA_ERR_UNSUPPORTED: the call is one for the scan kernels.  Without a workspace the whole sequence is one
@@ -557,25 +584,23 @@ int64_t fp32_chunk_fwd_workspace(int64_t B, int64_t N, int64_t H, int64_t D, int
 int launch_fp32_chunk_fwd(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb, int64_t ld_sn,
                           int64_t ld_sh, const float *s0, void *o, float *s_fin, void *workspace, int64_t workspace_bytes,
                           int B, int N, int H, int D, int E, int dtype, int ld_act, cudaStream_t st) {
-  if (!takes(B, N, H, D, E)) return LA_ERR_UNSUPPORTED;
+  const Plan p = plan_of(B, N, H, D, E, workspace != nullptr);
+  if (p.per == 0) return LA_ERR_UNSUPPORTED;
   // one 16-byte aligned row start per tensor
   const uintptr_t rows = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                          reinterpret_cast<uintptr_t>(o);
   const uintptr_t states = reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(s_fin);
   if ((rows & (dtype == LA_F32 ? 15u : 7u)) != 0 || (states & 15u) != 0) return LA_ERR_UNSUPPORTED;
-  const int64_t need = fp32_chunk_fwd_workspace(B, N, H, D, E);
-  const bool cut = need > 0 && workspace != nullptr;
-  if (cut && workspace_bytes < need) return LA_ERR_WORKSPACE;
-  if (cut && (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return LA_ERR_MISALIGNED;
-  const int chunks = (N + kC - 1) / kC;
+  const int64_t need = plan_bytes(p, (int64_t)B * H, D, E);
+  if (need > 0 && workspace_bytes < need) return LA_ERR_WORKSPACE;
+  if (need > 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return LA_ERR_MISALIGNED;
   Args a = {};
   a.q = q; a.k = k; a.v = v; a.ld = ld; a.ld_sb = ld_sb; a.ld_sn = ld_sn; a.ld_sh = ld_sh;
   a.s0 = s0; a.s_fin = s_fin; a.o = o;
   a.B = B; a.N = N; a.H = H; a.D = D; a.E = E; a.ld_act = ld_act;
-  const int per = cut ? chunks_per_segment(B, N, H) : chunks;
-  a.nseg = (chunks + per - 1) / per;
-  a.seg_tokens = per * kC;
-  if (cut) {
+  a.nseg = p.nseg;
+  a.seg_tokens = p.per * kC;
+  if (need > 0) {
     a.seg_state = static_cast<float *>(workspace);
     a.seg_decay = a.seg_state + (int64_t)B * H * a.nseg * D * E;
   }
