@@ -87,8 +87,9 @@ template <typename T, int VEC> struct Pack {
   }
 };
 
-// resident CTAs per SM without spills (N = features per lane)
-template <bool BWD, bool POST, int N> constexpr int ctas_per_sm() {
+// resident CTAs per SM (almost) without spills (N = features per lane)
+template <typename T, bool BWD, bool POST, int N> constexpr int ctas_per_sm() {
+  if (N <= 4 && sizeof(T) == 2) return BWD ? 4 : 5;
   return N <= (BWD && POST ? 4 : 8) ? 3 : (N <= 8 ? 2 : 1);
 }
 
@@ -103,7 +104,7 @@ template <bool BWD, bool POST, int N> constexpr int ctas_per_sm() {
 // POST = false: no gate behind the norm (the backward then needs neither y nor the bias, which is
 // what lets a third CTA onto the SM).
 template <typename T, bool BWD, bool POST, int VEC, int LPG, int NP>
-__global__ void __launch_bounds__(kThreads, (ctas_per_sm<BWD, POST, VEC * NP>())) norm_gate_kernel(const NormArgs a) {
+__global__ void __launch_bounds__(kThreads, (ctas_per_sm<T, BWD, POST, VEC * NP>())) norm_gate_kernel(const NormArgs a) {
   typedef Pack<T, VEC> P;
   typedef typename P::R R;
   constexpr int N = VEC * NP, RPW = 32 / LPG;
@@ -273,8 +274,8 @@ int launch_cfg(const NormArgs &a, bool bwd, cudaStream_t st) {
   long long blocks = (a.rows + rows_per_cta - 1) / rows_per_cta;
   // one wave over all groups: each CTA ends with its gradient sums, so few CTAs that walk many rows
   const bool post = a.gate != nullptr && a.post;
-  const int resident = !bwd ? ctas_per_sm<false, true, VEC * NP>()
-                            : (post ? ctas_per_sm<true, true, VEC * NP>() : ctas_per_sm<true, false, VEC * NP>());
+  const int resident = !bwd ? ctas_per_sm<T, false, true, VEC * NP>()
+                            : (post ? ctas_per_sm<T, true, true, VEC * NP>() : ctas_per_sm<T, true, false, VEC * NP>());
   const long long cap = ((long long)sms[dev] * resident + a.G - 1) / a.G;
   if (blocks > cap) blocks = cap;
   dim3 grid((unsigned)blocks, (unsigned)a.G);
