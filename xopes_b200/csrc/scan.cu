@@ -332,20 +332,24 @@ __global__ void __launch_bounds__(256) dld_scalar_kernel(const float *slots_q, i
   constexpr int kTile = 256 * kDldRows;
   // this thread's tokens of the tile that ends at `hi`: hi - 1 - tid kDldRows - i, the latest first
   auto load = [&](int64_t hi, float (&v)[kDldRows]) {
+    const int64_t last = hi - 1 - tid * kDldRows;  // token of i = 0
+    const int64_t idx = (bidx * N + last) * H + h;
+    if (ONE) {
 #pragma unroll
-    for (int i = 0; i < kDldRows; ++i) {
-      const int64_t t = hi - 1 - tid * kDldRows - i;
-      v[i] = 0.f;
-      if (t >= t_begin) {
-        const int64_t idx = (bidx * N + t) * H + h;
-        if (ONE) {
-          v[i] = slots_q[idx] - slots_k[idx];
-        } else {
-          for (int s = 0; s < ntq; ++s) v[i] += slots_q[s * slot + idx];
-          for (int s = 0; s < ntk; ++s) v[i] -= slots_k[s * slot + idx];
-        }
-      }
+      for (int i = 0; i < kDldRows; ++i) v[i] = last - i >= t_begin ? slots_q[idx - (int64_t)i * H] - slots_k[idx - (int64_t)i * H] : 0.f;
+      return;
     }
+    // slots outside, tokens inside: the loads of a slot's tokens go out together
+#pragma unroll
+    for (int i = 0; i < kDldRows; ++i) v[i] = 0.f;
+    for (int s = 0; s < ntq; ++s)
+#pragma unroll
+      for (int i = 0; i < kDldRows; ++i)
+        if (last - i >= t_begin) v[i] += slots_q[s * slot + idx - (int64_t)i * H];
+    for (int s = 0; s < ntk; ++s)
+#pragma unroll
+      for (int i = 0; i < kDldRows; ++i)
+        if (last - i >= t_begin) v[i] -= slots_k[s * slot + idx - (int64_t)i * H];
   };
   float cur[kDldRows], nxt[kDldRows];
   if (t_end > t_begin) load(t_end, cur);
