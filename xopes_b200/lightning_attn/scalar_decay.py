@@ -19,6 +19,7 @@ Differences, all deliberate:
     kernels apply the activation where they read the decay and the gradient returned for ld is
     d/dx.  Same result as passing F.logsigmoid(x), without the two elementwise passes.
 """
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -92,6 +93,12 @@ def _segmentation(lib, q, ld32, strides, cu, b, n, h, d, e, flags):
     return None
 
 
+@functools.lru_cache(maxsize=256)
+def _fwd_workspace_bytes(device_index, b, n, h, d, e, m, dtype, flags):
+    """The library's answer follows from the sizes and the device's SM count (1.3 us less per call)."""
+    return _lib.load().la_lasd_fwd_workspace_bytes(b, n, h, d, e, m, dtype, flags)
+
+
 class LasdFunction(torch.autograd.Function):
     """forward(q, k, v, ld, initial_state, cu_seqlens, flags) -> (o, final_state)."""
 
@@ -130,7 +137,7 @@ class LasdFunction(torch.autograd.Function):
         ws, ws_bytes = None, 0
         with _lib.device_of(q):
             if n < 128 or q.dtype == torch.float32:  # the fp32 CUDA-core path: states of its segments
-                ws_bytes = lib.la_lasd_fwd_workspace_bytes(b, n, h, d, e, m, _lib.dtype_code(q), flags)
+                ws_bytes = _fwd_workspace_bytes(q.device.index, b, n, h, d, e, m, _lib.dtype_code(q), flags)
                 if ws_bytes:
                     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
             rc = lib.la_lasd_fwd_ws(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
