@@ -13,9 +13,12 @@ def _call(n, h, strong, seed):
     return q, k, v, ldk
 
 
-def test_vector_decay_calls_overlap():
+@pytest.mark.parametrize("graphs", [False, True])
+def test_vector_decay_calls_overlap(graphs):
+    """graphs: a stream's calls are replayed from a graph, back to back, so that those of the streams interleave
+    densely."""
     from xopes_b200 import lightning_attn_func
-    n, h, rounds = 1024, 8, 100
+    n, h, rounds = 512, 4, 40
     inputs = [_call(n, h, False, 0), _call(n, h, True, 1), _call(n, h, True, 2), _call(n, h, False, 3)]
 
     def call(x):
@@ -25,15 +28,33 @@ def test_vector_decay_calls_overlap():
     ref = [call(x) for x in inputs]
     streams = [torch.cuda.Stream() for _ in inputs]
     torch.cuda.synchronize()
-    for s in streams:  # outputs that a call leaves unwritten are NaN
-        with torch.cuda.stream(s):
-            torch.full((rounds * n * h * 128,), float("nan"), dtype=torch.bfloat16, device="cuda")
-    torch.cuda.synchronize()
     out = [[] for _ in inputs]
-    for _ in range(rounds):
-        for x, s, o in zip(inputs, streams, out):
-            with torch.cuda.stream(s):
-                o.append(call(x))
-    torch.cuda.synchronize()
-    wrong = [sum(not torch.equal(r, o) for o in os) for r, os in zip(ref, out)]
+    if graphs:
+        held = []
+        for x, o in zip(inputs, out):
+            held.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(held[-1]):
+                o.extend(call(x) for _ in range(rounds))
+    wrong = [0] * len(inputs)
+    for _ in range(5):
+        if graphs:
+            for os in out:  # outputs that a call leaves unwritten stay NaN
+                for o in os:
+                    o.fill_(float("nan"))
+            torch.cuda.synchronize()
+            for g, s in zip(held, streams):
+                with torch.cuda.stream(s):
+                    g.replay()
+        else:
+            out = [[] for _ in inputs]
+            for s in streams:
+                with torch.cuda.stream(s):
+                    torch.full((rounds * n * h * 128 * 2,), float("nan"), dtype=torch.bfloat16, device="cuda")
+            for _ in range(rounds):
+                for x, s, o in zip(inputs, streams, out):
+                    with torch.cuda.stream(s):
+                        o.append(call(x))
+        torch.cuda.synchronize()
+        for i, (r, os) in enumerate(zip(ref, out)):
+            wrong[i] += sum(not torch.equal(r, o) for o in os)
     assert wrong == [0] * len(inputs)
