@@ -10,7 +10,9 @@
  * (cudaMallocFromPoolAsync / cudaFreeAsync on the caller's stream, about 10 MB per launch in
  * flight; under stream capture these become allocation nodes of the graph), and two non-blocking
  * side streams with three events on which independent gradient
- * passes of one backward call run beside each other.  la_lasd_bwd_noalloc uses neither.  The
+ * passes of one backward call run beside each other.  la_lasd_bwd_noalloc uses neither.  Both may be
+ * made under stream capture; the first call on a device that runs tcgen05 kernels may not (its
+ * device variables are looked up then: LA_ERR_CUDA, and the capture is lost).  The
  * return value is LA_OK or a negative LA_ERR_* code; la_status_string() turns it into text.
  *
  * Tensor layout (same as the reference operators): q, k are (B, N, H, D), v, o are (B, N, H, E),

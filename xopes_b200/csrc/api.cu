@@ -85,6 +85,7 @@ SideStream *side_stream() {
   std::lock_guard<std::mutex> lock(init_mu);
   SideStream &s = side[dev];
   if (!s.ready && !s.failed) {
+    CaptureRelaxed relaxed;
     if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&s.stream2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&s.fork_ev, cudaEventDisableTiming) != cudaSuccess ||

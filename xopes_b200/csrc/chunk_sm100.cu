@@ -1191,6 +1191,7 @@ cudaMemPool_t handoff_pool(DeviceInfo *d) {
   std::lock_guard<std::mutex> lock(g_info_mu);
   if (!d->pool_tried) {
     d->pool_tried = true;
+    CaptureRelaxed relaxed;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.handleTypes = cudaMemHandleTypeNone;

@@ -39,6 +39,14 @@ static inline int launch_status() {
   return e == cudaSuccess ? LA_OK : LA_ERR_CUDA;
 }
 
+// While one of these lives, calls that a stream capture forbids on its thread (making a pool, a stream or an
+// event) are allowed: for what the library makes once, on first need, which may be in a capture.
+struct CaptureRelaxed {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Address (on the current device) of the watchdog word that la_device_status() reads.
 // Defined in api.cu; kernels that can time out receive it as a parameter.
 int *status_word_ptr();
