@@ -30,8 +30,8 @@
 // at full load (4,800 with few CTAs); HBM would allow 2.9 us with 148 CTAs, the period is 3.2 us.
 // Next comes instruction fetch: a quarter of the SM's instruction-cache requests missed when the
 // loop was larger, which is why loops over pieces stay rolled where that costs nothing.
-// Forward / dq / dk and dv launches, 8 x 32 pairs of 8192 tokens: 394 / 387 / 726 us with one group of eight
-// warps, 366 / 358 / 668 us now; with a log-decay gradient (24 documents in 32768 tokens, 16 heads):
+// Forward / dq / dk and dv launches, 8 x 32 pairs of 8192 tokens, at an SM clock of 1,965 MHz: 394 / 387 / 726 us with one
+// group of eight warps, 366 / 358 / 668 us now; with a log-decay gradient (24 documents in 32768 tokens, 16 heads):
 // dq 256 -> 174 us, dk and dv 491 -> 354 us.
 //
 // Every mbarrier wait is bounded (sm100_ptx.cuh: mbar_wait); a wait that runs out sets the device
@@ -120,18 +120,17 @@ static_assert(offsetof(Small, cs) % 16 == 0 && offsetof(Small, bs) % 16 == 0, "v
 static_assert(kOffSmall % 16 == 0, "small area must start 16-byte aligned");
 
 struct ChunkArgs {
-  const void *xrow;
   float *rowdot;
   void *out;
   const float *ld;
   long long ld_sb, ld_sn, ld_sh;
   const float *t0;
   float *tfinal;
-  int state_transposed, reverse;
+  int state_transposed;
   const long long *cu;
   int B, N, H, M;
   int ld_act;  // 1: ld holds pre-activations x and the log decay is logsigmoid(x)
-  int fx, fz;  // features of X and Y (the contraction of X Y^T) and of Z, the output and xrow; <= 128
+  int fx, fz;  // features of X and Y (the contraction of X Y^T) and of Z, the output and the row-dot operand; <= 128
   int *status;
 };
 
@@ -294,7 +293,8 @@ __device__ __forceinline__ uint32_t kslice(int ks) { return (uint32_t)(ks >> 2) 
 // chunks, the row-dot operand) look at the real widths.
 // ACT = true: ld holds pre-activations of a logsigmoid (an instantiation of its own: the extra
 // arithmetic sits on the decay scan at the top of every chunk, which the plain path should not carry).
-// REV: the direction (a.reverse).  SPLIT = true: at least one pass of the launch has a row-dot operand (a log-decay gradient was asked for).
+// REV: the direction.  SPLIT = true: at least one pass of the launch has a row-dot operand (a log-decay
+// gradient was asked for).
 template <typename T, bool F128, bool ACT, bool SPLIT, bool REV>
 __global__ void __launch_bounds__(kThreads, 1)
 chunk_pass_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Launch lp) {
@@ -1220,9 +1220,9 @@ int fill_pass(const ChunkPass &p, int dtype, PassMaps &m, ChunkArgs &a) {
   m.r = m.o;
   if (p.xrow != nullptr && (rc = make_map(&m.r, p.xrow, dtype, p.B, p.N, p.H, p.fz)) != LA_OK) return rc;
   if ((reinterpret_cast<uintptr_t>(p.t0) | reinterpret_cast<uintptr_t>(p.tfinal)) & 15u) return LA_ERR_MISALIGNED;
-  a.xrow = p.xrow; a.rowdot = p.xrow ? p.rowdot : nullptr; a.out = p.out;
+  a.rowdot = p.xrow ? p.rowdot : nullptr; a.out = p.out;
   a.ld = p.ld; a.ld_sb = p.ld_sb; a.ld_sn = p.ld_sn; a.ld_sh = p.ld_sh;
-  a.t0 = p.t0; a.tfinal = p.tfinal; a.state_transposed = p.state_transposed; a.reverse = p.reverse;
+  a.t0 = p.t0; a.tfinal = p.tfinal; a.state_transposed = p.state_transposed;
   a.cu = reinterpret_cast<const long long *>(p.cu);
   a.B = p.B; a.N = p.N; a.H = p.H; a.M = p.M;
   a.fx = p.fx; a.fz = p.fz;

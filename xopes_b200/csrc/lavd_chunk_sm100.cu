@@ -129,7 +129,7 @@ struct LavdArgs {
   int dld_add;        // both passes add to a zeroed buffer (TMA reduce / atomics): order-free
   const float *t0;
   float *tfinal;
-  int state_transposed, reverse;
+  int state_transposed;
   const long long *cu;
   int B, N, H, M;
   int *status;
@@ -293,7 +293,7 @@ __device__ __forceinline__ void rescale2_z(uint8_t *gbase, uint32_t zoff, uint32
   }
 }
 
-// REV: the direction (a.reverse), a template parameter for the sake of the code's size: the two directions'
+// REV: the direction, a template parameter for the sake of the code's size: the two directions'
 // branches side by side cost 1 to 2 % of a step in instruction fetch.
 template <typename T, bool TMODE, bool REF2, bool REV>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -1112,8 +1112,9 @@ lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // the one-reference kernels' range: the first 64 tokens of up to four (sequence, head) pairs, all
 // features, the same sums and the same limit as those kernels use.  Only a hint (they check every chunk
 // themselves): decays that are out of range everywhere, as unscaled logsigmoids are, are seen here for
-// a few microseconds instead of by a full set of passes (B 2, H 16, N 4096, forward + backward: 1.10 ms
-// before, 0.69 ms with the sample); decays that are in range pay those microseconds.
+// a few microseconds instead of by a full set of passes (B 2, H 16, N 4096, forward + backward: 1.06 ms
+// before, 0.63 ms with the sample); decays that are in range pay those microseconds (B 1, H 16, N 512, forward:
+// 50 us with a memset in its place, 53 us).
 template <typename LT>
 __global__ void __launch_bounds__(512) lavd_sample_kernel(const LT *ld, const long long *cu, int N, int H, int pairs,
                                                            int ld_act, float limit, int *unsafe) {
@@ -1155,7 +1156,7 @@ int launch_t(const LavdPass &p, int dtype, cudaStream_t stream) {
     return rc;
   LavdArgs a;
   a.out = p.out; a.xrow = p.xrow; a.dld = p.xrow ? p.dld : nullptr; a.dld_sub = p.dld_sub; a.dld_add = p.dld_add;
-  a.t0 = p.t0; a.tfinal = p.tfinal; a.state_transposed = p.state_transposed; a.reverse = p.reverse;
+  a.t0 = p.t0; a.tfinal = p.tfinal; a.state_transposed = p.state_transposed;
   a.cu = reinterpret_cast<const long long *>(p.cu);
   a.B = p.B; a.N = p.N; a.H = p.H; a.M = p.M;
   a.status = status_word_ptr();
