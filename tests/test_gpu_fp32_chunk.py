@@ -35,9 +35,11 @@ def test_fp32_chunk_forward(b, n, h, d, e, dtype):
         ro, rs = orc.lasd_forward(q, k, v, ld, state, acc=torch.float64)
         assert_close("o", ro.to(dtype) if dtype != torch.float32 else ro, o, tol)
         assert_close("state", rs, sf, tol)
-        if dtype == torch.float32:  # no further from 64 bits than the token-by-token kernel (1e-7: ulp noise)
+        if dtype == torch.float32:
+            # no further from 64 bits than the token-by-token kernel, give or take one rounding of the result
+            # (root mean square at most 2^-25 of it; largest measured here 1.7e-8 over errors of 6e-8 to 1.3e-7)
             o2, s2 = lasd_recurrence_cuda(*dev[:4], initial_state=None if state is None else dev[4])
-            assert rel_l2(ro, o) <= rel_l2(ro, o2) + 1e-7 and rel_l2(rs, sf) <= rel_l2(rs, s2) + 1e-7
+            assert rel_l2(ro, o) <= rel_l2(ro, o2) + 2 ** -25 and rel_l2(rs, sf) <= rel_l2(rs, s2) + 2 ** -25
 
 
 def test_fp32_chunk_forward_decay_forms():
