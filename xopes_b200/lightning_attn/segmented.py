@@ -77,15 +77,20 @@ def worth_segmenting(doc_bounds, h: int, cap: int, sms: int) -> bool:
       CTAs, and a sequence longer than one share then spans three of them - the middle one cannot
       start before the first has finished its part - so any such sequence is cut.
     * Few pairs (a quarter of the SMs or fewer): cut once a sequence is longer than 1.5 shares
-      (B = 1, H = 16, N = 32768 forward + backward: 0.56 ms against 1.48 ms).
+      (B = 1, H = 16, N = 32768 forward + backward: 0.51 ms against 1.25 ms).
     * In between the plain launch gives one CTA to each pair and lasts as long as its longest
-      sequence.  A CTA needs about 3 us per chunk at any occupancy, but with few pairs the
-      backward's launches run side by side on two streams, so idle SMs cost a forward + backward
-      step less than their count suggests; the effective cost per chunk and pass below is fitted to
-      measured steps on B200 (1.6 us with 32 pairs, 2.2 with 64, 3.3 with 128, 3.7 with every SM
-      busy).  Equal-length batches are left alone (48, 96, 128 pairs of N = 8192: cutting loses
-      7-27 %); the cut is taken only when the longest sequence makes the plain launch clearly longer
-      than the balanced one, as for the ragged documents of a sequence-parallel rank."""
+      sequence.  With few pairs the backward's launches run side by side on two streams, so idle SMs
+      cost a forward + backward step less than their count suggests.  Equal-length batches are left
+      alone (48, 96, 128 pairs of N = 8192, forward + backward: cutting loses 18, 25 and 51 %); the cut is
+      taken only when the longest sequence makes the plain launch clearly longer than the balanced
+      one, as for the ragged documents of a sequence-parallel rank.
+
+    The costs per chunk and pass (1.6 us with 32 pairs, 2.2 with 64, 3.3 with 128, 3.7 with every SM
+    busy) are fitted to steps of the chunk kernel as it was with one group of compute warps.  It now
+    takes 1.7 us with 32 pairs, 2.6 with 64, 3.0 with 96, 3.6 to 4.1 with 128, forward + backward at
+    N = 8192; the rule was not fitted again.  Where it is known to be off: 8 to 32 pairs of N = 2048 are
+    cut (69 us forward) although the plain launch takes 47, 64 pairs of N = 16384 are left alone (1.01 ms
+    forward + backward) although the cut takes 0.83."""
     chunks = [-(-(b - a) // 128) for a, b in doc_bounds]
     longest = max(chunks)
     if longest * 128 <= cap:
