@@ -89,7 +89,7 @@ template <typename T, int VEC> struct Pack {
 
 // resident CTAs per SM (almost) without spills (N = features per lane)
 template <typename T, bool BWD, bool POST, int N> constexpr int ctas_per_sm() {
-  if (N <= 4 && sizeof(T) == 2) return BWD ? 4 : 5;
+  if (N <= 4 && sizeof(T) == 2) return BWD ? 4 : 8;
   return N <= (BWD && POST ? 4 : 8) ? 3 : (N <= 8 ? 2 : 1);
 }
 
@@ -98,8 +98,10 @@ template <typename T, bool BWD, bool POST, int N> constexpr int ctas_per_sm() {
 // step are loaded before the current step is worked on.
 //
 // Bound by HBM: 75 MB forward / 126 MB backward at 16384 rows of 12 groups of 64 (bf16) are 11.5 / 19 us
-// at the measured copy bandwidth.  A whole warp per group left half its lanes idle at 64 features,
-// had one 8-byte load per operand in flight and sent one atomic per warp and feature.
+// at the measured copy bandwidth; 22 / 39 us here, 52 / 198 with a whole warp per group, which left half its
+// lanes idle at 64 features, had one 8-byte load per operand in flight and sent one atomic per warp and
+// feature.  Groups that are no multiple of 8 features have 4 a lane and more CTAs per SM: 100 features, 32768 rows
+// of 8 groups, 65 / 112 us (77 / 293 with a warp per group, 125 / 262 here with three CTAs).
 //
 // POST = false: no gate behind the norm (the backward then needs neither y nor the bias, which is
 // what lets a third CTA onto the SM).
@@ -108,6 +110,8 @@ __global__ void __launch_bounds__(kThreads, (ctas_per_sm<T, BWD, POST, VEC * NP>
   typedef Pack<T, VEC> P;
   typedef typename P::R R;
   constexpr int N = VEC * NP, RPW = 32 / LPG;
+  // the next rows are loaded ahead, except where eight CTAs per SM cover the latency and leave no registers for it
+  constexpr bool kAhead = BWD || N > 4 || sizeof(T) > 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gl = lane % LPG, sub = lane / LPG;
   const int g = blockIdx.y, e = a.e;
@@ -143,11 +147,12 @@ __global__ void __launch_bounds__(kThreads, (ctas_per_sm<T, BWD, POST, VEC * NP>
     }
   };
   const long long first = ((long long)blockIdx.x * kWarps + warp) * RPW;  // uniform over the warp
-  fetch(first + sub);
+  if (kAhead) fetch(first + sub);
   for (long long r0 = first; r0 < a.rows; r0 += step) {
     const long long r = r0 + sub;
     const bool live = r < a.rows;
     const long long off = r * stride + (long long)g * e;
+    if (!kAhead) fetch(r);
     float x[N], gt[N], d_o[N], act[N], dact[N], z[N];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
@@ -155,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, (ctas_per_sm<T, BWD, POST, VEC * NP>
       P::unpack(rg[p], gt + p * VEC);
       if (BWD) P::unpack(rd[p], d_o + p * VEC);
     }
-    fetch(r + step);
+    if (kAhead) fetch(r + step);
     if (has_gate) {
       activate<BWD, N>(gt, a.act, act, dact);
     } else {
