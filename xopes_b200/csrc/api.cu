@@ -624,6 +624,7 @@ int la_lavd_bwd(const void *q, const void *k, const void *v, const float *ldk, c
       v2.skip = q2.skip = k2.skip = nullptr;
       v2.unsafe = q2.unsafe = k2.unsafe = unsafe + 1;
       q2.dld_add = k2.dld_add = 0;
+      q2.both_ways = k2.both_ways = 0;
       int r2 = launch_lavd_pass(v2, dtype, s_v);
       if (r2 == LA_OK) r2 = launch_lavd_pass(q2, dtype, st);
       if (r2 == LA_OK) r2 = launch_lavd_pass(k2, dtype, st);
@@ -638,6 +639,7 @@ int la_lavd_bwd(const void *q, const void *k, const void *v, const float *ldk, c
       std::unique_lock<std::mutex> side_lock(side->mu);
       if (all3) {
         cq.dld_add = ck.dld_add = 1;
+        cq.both_ways = ck.both_ways = 1;
         if (cudaMemsetAsync(dldk, 0, (size_t)B * N * H * D * sizeof(float), st) != cudaSuccess) return LA_ERR_CUDA;
       }
       if (!side_fork(side, st) || (all3 && !side_fork2(side))) return LA_ERR_CUDA;

@@ -78,6 +78,7 @@ struct LavdPass {
   int ref2 = 0;
   const int *enable = nullptr;  // optional device word: the launch does nothing while it reads 0
   const int *skip = nullptr;    // optional device word: a CTA that finds it raised does nothing
+  int both_ways = 0;            // 1: a pass of the other direction (same mode) runs beside this one: use the code that serves both
 };
 // Clears unsafe[0..1] and raises unsafe[0] if a sample of the decays is out of the one-reference range.
 int launch_lavd_sample(const void *ldk, const int64_t *cu, int B, int N, int H, int M, int dtype, int ld16, int ld_act,

@@ -130,6 +130,7 @@ struct LavdArgs {
   const float *t0;
   float *tfinal;
   int state_transposed;
+  int reverse;        // read with DIR = kBothWays only
   const long long *cu;
   int B, N, H, M;
   int *status;
@@ -293,9 +294,12 @@ __device__ __forceinline__ void rescale2_z(uint8_t *gbase, uint32_t zoff, uint32
   }
 }
 
-// REV: the direction, a template parameter for the sake of the code's size: the two directions'
-// branches side by side cost 1 to 2 % of a step in instruction fetch.
-template <typename T, bool TMODE, bool REF2, bool REV>
+// DIR: the direction (0 forward, 1 reverse), a template parameter for the sake of the code's size: the two
+// directions' branches side by side cost 1 to 2 % of a step in instruction fetch.  2: a.reverse says, one code
+// for both; for a forward and a reverse pass that run beside each other, where two codes (and a third for dv)
+// cost more than the branches: 16 pairs of 8192 tokens, forward + backward, 1.09 ms with two, 1.02 with one.
+constexpr int kBothWays = 2;
+template <typename T, bool TMODE, bool REF2, int DIR>
 __global__ void __launch_bounds__(kThreads, 1)
 lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                  const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_ld,
@@ -324,7 +328,7 @@ lavd_pass_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   }
   const int len = (int)(t_end - t_begin);
   const int nc = (len + kChunk - 1) / kChunk;
-  constexpr bool rev = REV;
+  const bool rev = DIR == kBothWays ? a.reverse != 0 : DIR == 1;
 
   const uint32_t full_ck = smem_u32(&sm->full_ck), full_yz = smem_u32(&sm->full_yz), full_x = smem_u32(&sm->full_x);
   const uint32_t empty_ck = smem_u32(&sm->empty_ck), empty_yz = smem_u32(&sm->empty_yz), empty_x = smem_u32(&sm->empty_x);
@@ -1156,7 +1160,7 @@ int launch_t(const LavdPass &p, int dtype, cudaStream_t stream) {
     return rc;
   LavdArgs a;
   a.out = p.out; a.xrow = p.xrow; a.dld = p.xrow ? p.dld : nullptr; a.dld_sub = p.dld_sub; a.dld_add = p.dld_add;
-  a.t0 = p.t0; a.tfinal = p.tfinal; a.state_transposed = p.state_transposed;
+  a.t0 = p.t0; a.tfinal = p.tfinal; a.state_transposed = p.state_transposed; a.reverse = p.reverse;
   a.cu = reinterpret_cast<const long long *>(p.cu);
   a.B = p.B; a.N = p.N; a.H = p.H; a.M = p.M;
   a.status = status_word_ptr();
@@ -1166,7 +1170,10 @@ int launch_t(const LavdPass &p, int dtype, cudaStream_t stream) {
   a.ld_act = p.ld_act;
   a.ld16 = p.ld16;
   if (a.status == nullptr || a.unsafe == nullptr) return LA_ERR_CUDA;
-  auto kern = p.reverse ? lavd_pass_kernel<T, TMODE, REF2, true> : lavd_pass_kernel<T, TMODE, REF2, false>;
+  auto kern = p.reverse ? lavd_pass_kernel<T, TMODE, REF2, 1> : lavd_pass_kernel<T, TMODE, REF2, 0>;
+  if constexpr (TMODE && !REF2) {
+    if (p.both_ways) kern = lavd_pass_kernel<T, TMODE, REF2, kBothWays>;
+  }
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
     return LA_ERR_CUDA;
   const int nb = p.cu ? p.M : p.B;
