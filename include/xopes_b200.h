@@ -8,7 +8,8 @@
  * itself, once per device and on first need: a stream-ordered memory pool from which a tcgen05
  * launch that splits (sequence, head) pairs across CTAs takes its hand-off scratch
  * (cudaMallocFromPoolAsync / cudaFreeAsync on the caller's stream, about 10 MB per launch in
- * flight; under stream capture these become allocation nodes of the graph), and two non-blocking
+ * flight) and la_lasd_fwd the states of its segments on the fp32 path (at most 2 x SMs + B H of
+ * D x E floats; under stream capture both become allocation nodes of the graph), and two non-blocking
  * side streams with three events on which independent gradient
  * passes of one backward call run beside each other.  la_lasd_bwd_noalloc uses neither.  Both may be
  * made under stream capture; the first call on a device that runs tcgen05 kernels may not (its
@@ -123,11 +124,12 @@ LA_API int la_lasd_fwd(const void *q, const void *k, const void *v, const float 
 /* la_lasd_fwd with scratch from the caller, for the fp32 CUDA-core path (la_lasd_path 0).  Without
  * cu_seqlens and LA_FLAG_FORCE_RECURRENCE, with D and E multiples of 4 up to 128, N >= 16 and aligned
  * tensors (16 bytes for fp32 and the states, 8 for 16-bit) that path's forward runs in chunks of 64 tokens
- * where sizes and the SM count say that this is quicker than token by token.
- * Given la_lasd_fwd_workspace_bytes bytes (16-byte aligned) the chunks of few (sequence, head) pairs run
- * side by side; with workspace NULL, as in la_lasd_fwd, each pair walks its chunks in turn, which takes no
- * scratch and rounds differently.  Other calls need 0 bytes and ignore the workspace.  The kernels are
- * chosen from the arguments alone, the same under stream capture, and nothing here allocates on this path.
+ * where sizes and the SM count say that this is quicker than token by token, the chunks of few (sequence,
+ * head) pairs side by side.  That takes la_lasd_fwd_workspace_bytes bytes of scratch (0: none, as for every
+ * other call).  la_lasd_fwd takes them from the library's pool; la_lasd_fwd_ws takes them as an argument
+ * (16-byte aligned) and allocates nothing on this path, with the same results to the bit.  With workspace
+ * NULL each pair walks its chunks in turn, without scratch and rounded differently, as la_lasd_fwd does where
+ * the pool has no memory.  Which kernels run does not depend on earlier calls or on stream capture.
  * LA_ERR_WORKSPACE / LA_ERR_MISALIGNED: a workspace that is too small or not aligned. */
 LA_API int64_t la_lasd_fwd_workspace_bytes(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E,
                                     int64_t M, int dtype, unsigned flags);

@@ -159,6 +159,11 @@ def test_fp32_chunk_forward_workspace(b, n, h, d):
         assert call(at, nbytes) == 0
         assert_close("o", ro, o, TOL_FP32)
         assert_close("state", rs, sf, TOL_FP32)
+    call(ws.data_ptr(), need)
+    o2, s2 = torch.empty_like(o), torch.empty_like(sf)  # scratch from the library's pool: the same to the bit
+    assert lib.la_lasd_fwd(*(t.data_ptr() for t in dev[:4]), *dev[3].stride(), dev[4].data_ptr(), None, o2.data_ptr(),
+                           s2.data_ptr(), b, n, h, d, d, 0, _lib.LA_F32, 0, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(o, o2) and torch.equal(sf, s2)
     if need:
         assert call(ws.data_ptr(), need - 1) == -7 and call(ws.data_ptr() + 8, need) == -6
         assert torch.isnan(o).all()

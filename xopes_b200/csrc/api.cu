@@ -250,28 +250,12 @@ int la_debug_umma_probe(int variant, const void *a, const void *b, float *d, int
 // ------------------------------------------------------------------------------------------------
 // scalar decay
 // ------------------------------------------------------------------------------------------------
-int64_t la_lasd_fwd_workspace_bytes(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E, int64_t M, int dtype,
-                                    unsigned flags) {
-  if (B <= 0 || N <= 0 || H <= 0 || D <= 0 || E <= 0 || M != 0 || (flags & LA_FLAG_FORCE_RECURRENCE) ||
-      la_lasd_path(N, D, E, dtype, flags) != 0)
-    return 0;
-  return fp32_chunk_fwd_workspace(B, N, H, D, E);
-}
-
-int la_lasd_fwd(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb,
-                int64_t ld_sn, int64_t ld_sh, const float *initial_state,
-                const int64_t *cu_seqlens, void *o, float *final_state, int64_t B, int64_t N,
-                int64_t H, int64_t D, int64_t E, int64_t M, int dtype, unsigned flags,
-                void *stream) {
-  return la_lasd_fwd_ws(q, k, v, ld, ld_sb, ld_sn, ld_sh, initial_state, cu_seqlens, o, final_state, nullptr, 0, B, N,
-                        H, D, E, M, dtype, flags, stream);
-}
-
-int la_lasd_fwd_ws(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb,
-                   int64_t ld_sn, int64_t ld_sh, const float *initial_state,
-                   const int64_t *cu_seqlens, void *o, float *final_state, void *workspace,
-                   int64_t workspace_bytes, int64_t B, int64_t N, int64_t H, int64_t D, int64_t E,
-                   int64_t M, int dtype, unsigned flags, void *stream) {
+// use_pool: the fp32 chunk form may take scratch from the library's pool
+static int lasd_fwd_impl(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb,
+                         int64_t ld_sn, int64_t ld_sh, const float *initial_state, const int64_t *cu_seqlens,
+                         void *o, float *final_state, void *workspace, int64_t workspace_bytes, int use_pool,
+                         int64_t B, int64_t N, int64_t H, int64_t D, int64_t E, int64_t M, int dtype,
+                         unsigned flags, void *stream) {
   int rc = check_common(q, k, v, B, N, H, D, E, M, cu_seqlens, dtype);
   if (rc != LA_OK) return rc;
   if (o == nullptr || ld == nullptr) return LA_ERR_NULL_POINTER;
@@ -297,11 +281,37 @@ int la_lasd_fwd_ws(const void *q, const void *k, const void *v, const float *ld,
   // explicit request for the recurrence run token by token.
   if (!(flags & LA_FLAG_FORCE_RECURRENCE) && cu_seqlens == nullptr) {
     rc = launch_fp32_chunk_fwd(q, k, v, ld, ld_sb, ld_sn, ld_sh, initial_state, o, final_state, workspace,
-                               workspace_bytes, s.B, s.N, s.H, s.D, s.E, dtype, ld_act, st);
+                               workspace_bytes, use_pool, s.B, s.N, s.H, s.D, s.E, dtype, ld_act, st);
     if (rc != LA_ERR_UNSUPPORTED) return rc;
   }
   return scan_forward(s, q, k, v, ld, ld_sb, ld_sn, ld_sh, nullptr, nullptr, initial_state, o,
                       final_state, dtype, st, nullptr, ld_act);
+}
+
+int64_t la_lasd_fwd_workspace_bytes(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E, int64_t M, int dtype,
+                                    unsigned flags) {
+  if (B <= 0 || N <= 0 || H <= 0 || D <= 0 || E <= 0 || M != 0 || (flags & LA_FLAG_FORCE_RECURRENCE) ||
+      la_lasd_path(N, D, E, dtype, flags) != 0)
+    return 0;
+  return fp32_chunk_fwd_workspace(B, N, H, D, E);
+}
+
+int la_lasd_fwd(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb,
+                int64_t ld_sn, int64_t ld_sh, const float *initial_state,
+                const int64_t *cu_seqlens, void *o, float *final_state, int64_t B, int64_t N,
+                int64_t H, int64_t D, int64_t E, int64_t M, int dtype, unsigned flags,
+                void *stream) {
+  return lasd_fwd_impl(q, k, v, ld, ld_sb, ld_sn, ld_sh, initial_state, cu_seqlens, o, final_state, nullptr, 0, 1, B, N,
+                       H, D, E, M, dtype, flags, stream);
+}
+
+int la_lasd_fwd_ws(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb,
+                   int64_t ld_sn, int64_t ld_sh, const float *initial_state,
+                   const int64_t *cu_seqlens, void *o, float *final_state, void *workspace,
+                   int64_t workspace_bytes, int64_t B, int64_t N, int64_t H, int64_t D, int64_t E,
+                   int64_t M, int dtype, unsigned flags, void *stream) {
+  return lasd_fwd_impl(q, k, v, ld, ld_sb, ld_sn, ld_sh, initial_state, cu_seqlens, o, final_state, workspace,
+                       workspace_bytes, 0, B, N, H, D, E, M, dtype, flags, stream);
 }
 
 // Workspace layout: [recomputed final state, rounded up to 16 bytes][row dots of q.dq][row dots of

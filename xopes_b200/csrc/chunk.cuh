@@ -32,16 +32,19 @@ struct ChunkPass {
   int no_scratch = 0;  // 1: never take hand-off scratch from the library's pool (one CTA per pair)
 };
 
-// SM count of the current device (0 on error).
+// SM count of the current device (0 on error) and scratch in stream order from the pool the library
+// owns (free it with cudaFreeAsync on the same stream).
 int device_sms();
+int scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
 
 // Chunk-parallel scalar-decay forward in fp32 arithmetic (chunk_fp32.cu), without cu_seqlens; returns
-// LA_ERR_UNSUPPORTED for a call that belongs to the scan kernels.  The workspace (fp32_chunk_fwd_workspace
-// bytes, possibly 0) holds the states of the segments; without one the sequence is not cut.
+// LA_ERR_UNSUPPORTED for a call that belongs to the scan kernels.  The states of the segments are held in the
+// workspace (fp32_chunk_fwd_workspace bytes, possibly 0) or, with use_pool, in scratch from the pool; with
+// neither the sequence is not cut.
 int64_t fp32_chunk_fwd_workspace(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E);
 int launch_fp32_chunk_fwd(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb, int64_t ld_sn,
                           int64_t ld_sh, const float *s0, void *o, float *s_fin, void *workspace, int64_t workspace_bytes,
-                          int B, int N, int H, int D, int E, int dtype, int ld_act, cudaStream_t st);
+                          int use_pool, int B, int N, int H, int D, int E, int dtype, int ld_act, cudaStream_t st);
 
 bool chunk_supported(int64_t N, int64_t D, int64_t E, int dtype);
 // With more (sequence, head) pairs than SMs the launch runs one CTA per SM on an even split of

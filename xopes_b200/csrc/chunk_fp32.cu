@@ -543,7 +543,8 @@ struct Plan {
 // costs at most 1.24 times the chunk form's time (32 tokens of 192 pairs of 16 features, 21 us).
 Plan plan_of(int64_t B, int64_t N, int64_t H, int64_t D, int64_t E, bool scratch) {
   if (D > 128 || E > 128 || D % 4 != 0 || E % 4 != 0 || N < 16 || B * H > 65535) return {0, 0};
-  const int64_t pairs = B * H, chunks = (N + kC - 1) / kC, sms = device_sms() > 0 ? device_sms() : 1;
+  const int dev_sms = device_sms();
+  const int64_t pairs = B * H, chunks = (N + kC - 1) / kC, sms = dev_sms > 0 ? dev_sms : 1;
   // with scratch, as many segments as keep about two CTAs per SM (the states of the segments are then at most
   // 2 x SMs + B H of D x E floats, whatever N is)
   int64_t parts = scratch ? (2 * sms + pairs - 1) / pairs : 1;
@@ -579,37 +580,48 @@ int64_t fp32_chunk_fwd_workspace(int64_t B, int64_t N, int64_t H, int64_t D, int
   return plan_bytes(plan_of(B, N, H, D, E, true), B * H, D, E);
 }
 
-// LA_ERR_UNSUPPORTED: the call is one for the scan kernels.  Without a workspace the whole sequence is one
-// segment: no scratch, one launch.
+// LA_ERR_UNSUPPORTED: the call is one for the scan kernels.  With neither a workspace nor the pool (or where that
+// has no memory) the whole sequence is one segment: no scratch, one launch.
 int launch_fp32_chunk_fwd(const void *q, const void *k, const void *v, const float *ld, int64_t ld_sb, int64_t ld_sn,
                           int64_t ld_sh, const float *s0, void *o, float *s_fin, void *workspace, int64_t workspace_bytes,
-                          int B, int N, int H, int D, int E, int dtype, int ld_act, cudaStream_t st) {
-  const Plan p = plan_of(B, N, H, D, E, workspace != nullptr);
-  if (p.per == 0) return LA_ERR_UNSUPPORTED;
+                          int use_pool, int B, int N, int H, int D, int E, int dtype, int ld_act, cudaStream_t st) {
   // one 16-byte aligned row start per tensor
   const uintptr_t rows = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                          reinterpret_cast<uintptr_t>(o);
   const uintptr_t states = reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(s_fin);
   if ((rows & (dtype == LA_F32 ? 15u : 7u)) != 0 || (states & 15u) != 0) return LA_ERR_UNSUPPORTED;
-  const int64_t need = plan_bytes(p, (int64_t)B * H, D, E);
-  if (need > 0 && workspace_bytes < need) return LA_ERR_WORKSPACE;
-  if (need > 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return LA_ERR_MISALIGNED;
+  const int64_t pairs = (int64_t)B * H;
+  Plan p = plan_of(B, N, H, D, E, workspace != nullptr || use_pool);
+  void *scratch = workspace, *pooled = nullptr;
+  if (plan_bytes(p, pairs, D, E) > 0) {
+    if (workspace != nullptr) {
+      if (workspace_bytes < plan_bytes(p, pairs, D, E)) return LA_ERR_WORKSPACE;
+      if ((reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return LA_ERR_MISALIGNED;
+    } else if (scratch_alloc(&pooled, (size_t)plan_bytes(p, pairs, D, E), st) == LA_OK) {
+      scratch = pooled;
+    } else {
+      p = plan_of(B, N, H, D, E, false);
+    }
+  }
+  if (p.per == 0) return LA_ERR_UNSUPPORTED;
   Args a = {};
   a.q = q; a.k = k; a.v = v; a.ld = ld; a.ld_sb = ld_sb; a.ld_sn = ld_sn; a.ld_sh = ld_sh;
   a.s0 = s0; a.s_fin = s_fin; a.o = o;
   a.B = B; a.N = N; a.H = H; a.D = D; a.E = E; a.ld_act = ld_act;
   a.nseg = p.nseg;
   a.seg_tokens = p.per * kC;
-  if (need > 0) {
-    a.seg_state = static_cast<float *>(workspace);
-    a.seg_decay = a.seg_state + (int64_t)B * H * a.nseg * D * E;
+  if (p.nseg > 1) {
+    a.seg_state = static_cast<float *>(scratch);
+    a.seg_decay = a.seg_state + pairs * a.nseg * D * E;
   }
+  int rc = LA_ERR_UNSUPPORTED;
   switch (dtype) {
-    case LA_F32: return launch_t<float>(a, st);
-    case LA_BF16: return launch_t<__nv_bfloat16>(a, st);
-    case LA_F16: return launch_t<__half>(a, st);
+    case LA_F32: rc = launch_t<float>(a, st); break;
+    case LA_BF16: rc = launch_t<__nv_bfloat16>(a, st); break;
+    case LA_F16: rc = launch_t<__half>(a, st); break;
   }
-  return LA_ERR_UNSUPPORTED;
+  if (pooled != nullptr && cudaFreeAsync(pooled, st) != cudaSuccess && rc == LA_OK) rc = LA_ERR_CUDA;
+  return rc;
 }
 
 }  // namespace la

@@ -1452,6 +1452,16 @@ int device_sms() {
   return di != nullptr ? di->sms : 0;
 }
 
+int scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream) {
+  *ptr = nullptr;
+  DeviceInfo *di = device_info();
+  cudaMemPool_t pool = di != nullptr ? handoff_pool(di) : nullptr;
+  if (pool != nullptr && cudaMallocFromPoolAsync(ptr, bytes, pool, stream) == cudaSuccess) return LA_OK;
+  cudaGetLastError();
+  *ptr = nullptr;
+  return LA_ERR_CUDA;
+}
+
 int umma_probe(int variant, const void *a, const void *b, float *d, int dtype, cudaStream_t stream) {
   if (a == nullptr || b == nullptr || d == nullptr) return LA_ERR_NULL_POINTER;
   if (variant < 0 || variant > 4) return LA_ERR_BAD_SHAPE;

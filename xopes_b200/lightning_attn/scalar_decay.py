@@ -19,7 +19,6 @@ Differences, all deliberate:
     kernels apply the activation where they read the decay and the gradient returned for ld is
     d/dx.  Same result as passing F.logsigmoid(x), without the two elementwise passes.
 """
-import functools
 from typing import Optional, Tuple
 
 import torch
@@ -93,12 +92,6 @@ def _segmentation(lib, q, ld32, strides, cu, b, n, h, d, e, flags):
     return None
 
 
-@functools.lru_cache(maxsize=256)
-def _fwd_workspace_bytes(device_index, b, n, h, d, e, m, dtype, flags):
-    """The library's answer follows from the sizes and the device's SM count (1.3 us less per call)."""
-    return _lib.load().la_lasd_fwd_workspace_bytes(b, n, h, d, e, m, dtype, flags)
-
-
 class LasdFunction(torch.autograd.Function):
     """forward(q, k, v, ld, initial_state, cu_seqlens, flags) -> (o, final_state)."""
 
@@ -134,15 +127,20 @@ class LasdFunction(torch.autograd.Function):
             return o, sf
         o = torch.empty(b, n, h, e, dtype=q.dtype, device=q.device)
         sf = torch.empty(nb, h, d, e, dtype=torch.float32, device=q.device)
-        ws, ws_bytes = None, 0
+        dtype, ws_bytes = _lib.dtype_code(q), 0
         with _lib.device_of(q):
-            if n < 128 or q.dtype == torch.float32:  # the fp32 CUDA-core path: states of its segments
-                ws_bytes = _fwd_workspace_bytes(q.device.index, b, n, h, d, e, m, _lib.dtype_code(q), flags)
-                if ws_bytes:
-                    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-            rc = lib.la_lasd_fwd_ws(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
-                                    _lib.ptr(s0), _lib.ptr(cu), _lib.ptr(o), _lib.ptr(sf), _lib.ptr(ws), ws_bytes,
-                                    b, n, h, d, e, m, _lib.dtype_code(q), flags, _lib.stream_of(q))
+            if (n < 128 or dtype == _lib.LA_F32) and torch._C._cuda_isCurrentStreamCapturing():
+                # scratch of the fp32 path out of the graph's memory instead of allocation nodes in the graph
+                ws_bytes = lib.la_lasd_fwd_workspace_bytes(b, n, h, d, e, m, dtype, flags)
+            if ws_bytes:
+                ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+                rc = lib.la_lasd_fwd_ws(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
+                                        _lib.ptr(s0), _lib.ptr(cu), _lib.ptr(o), _lib.ptr(sf), _lib.ptr(ws), ws_bytes,
+                                        b, n, h, d, e, m, dtype, flags, _lib.stream_of(q))
+            else:
+                rc = lib.la_lasd_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(ld32), sb, sn, sh,
+                                     _lib.ptr(s0), _lib.ptr(cu), _lib.ptr(o), _lib.ptr(sf),
+                                     b, n, h, d, e, m, dtype, flags, _lib.stream_of(q))
         _lib.check(rc, "la_lasd_fwd")
         ctx.save_for_backward(q, k, v, ld, s0, cu, None)
         ctx.flags = flags
