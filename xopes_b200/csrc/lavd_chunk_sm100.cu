@@ -297,7 +297,7 @@ __device__ __forceinline__ void rescale2_z(uint8_t *gbase, uint32_t zoff, uint32
 // DIR: the direction (0 forward, 1 reverse), a template parameter for the sake of the code's size: the two
 // directions' branches side by side cost 1 to 2 % of a step in instruction fetch.  2: a.reverse says, one code
 // for both; for a forward and a reverse pass that run beside each other, where two codes (and a third for dv)
-// cost more than the branches: 16 pairs of 8192 tokens, forward + backward, 1.09 ms with two, 1.02 with one.
+// cost more than the branches: 16 pairs of 8192 tokens, forward + backward, 1.08 ms with two, 1.00 with one.
 constexpr int kBothWays = 2;
 template <typename T, bool TMODE, bool REF2, int DIR>
 __global__ void __launch_bounds__(kThreads, 1)
